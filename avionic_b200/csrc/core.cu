@@ -36,6 +36,7 @@
 #include "radial.cuh"
 #include "tc_dft.cuh"
 #include "utils_kernels.cuh"
+#include "yfft.cuh"
 
 
 
@@ -264,6 +265,7 @@ avx_status configure_once() {
   AVX_CK(avx::configure_radial_kernels());
   AVX_CK(avx::configure_fft2d_kernels());
   AVX_CK(avx::configure_tc_kernels());
+  AVX_CK(avx::configure_yfft_kernels());
   g_configured |= bit;
   return AVX_OK;
 }
@@ -311,7 +313,11 @@ struct avx_operator {
   int dft_mode = AVX_DFT_FP32;
   int tc_np = 0;  // MMA N of the y-transform = MMA K of the column adjoint; 0: split form not available
   DevBuf<uint4> tc_ytab, tc_ctab;
-  DevBuf<float2> tc_b1t;  // coil maps in column-tile order for operator applies
+  DevBuf<float2> b1t;  // coil maps in the y-transforms' order, for operator applies
+  // register-FFT y-transforms (yfft.cuh); yf_n1 = 0: the height has no factor for them
+  int yf_n1 = 0, max_rows = 0;
+  DevBuf<int2> yf_order;
+  DevBuf<float2> yf_coef;
 
   CartGeomDev geom() const {
     CartGeomDev g;
@@ -379,24 +385,33 @@ static avx_status build_operator(avx_operator* op, const float* h_mask) {
     AVX_CK(op->d_mask.alloc((size_t)T * H * W));
     AVX_CK(cudaMemcpy(op->d_mask.p, h_mask, (size_t)T * H * W * sizeof(float), cudaMemcpyHostToDevice));
   }
-  // coefficient tables of the tensor-core transforms (at most 48 rows per frame)
   int max_rows = 0;
   for (int t = 0; t < T; ++t) max_rows = std::max(max_rows, op->row_off[t + 1] - op->row_off[t]);
+  op->max_rows = max_rows;
   const int np = std::max(16, (2 * max_rows + 15) / 16 * 16);
-  op->tc_np = 0;
-  op->dft_mode = AVX_DFT_FP32;
-  if (max_rows > 0 && np <= TC_MAX_NP) {
+  op->tc_np = max_rows > 0 && np <= TC_MAX_NP ? np : 0;
+  op->dft_mode = op->tc_np ? AVX_DFT_SPLIT_BF16X3 : AVX_DFT_FP32;
+  const int sy = op->centered ? H / 2 : 0;
+  op->yf_n1 = max_rows > 0 ? avx::yfft_n1(H, max_rows) : 0;
+  if (op->yf_n1) {
+    const int n1 = op->yf_n1;
+    std::vector<int2> order(op->R);
+    std::vector<float2> coef((size_t)op->R * (H / n1));
+    avx::yfft_build(H, T, sy, n1, op->rows.data(), op->row_off.data(), order.data(), coef.data());
+    AVX_CK(op->yf_order.alloc(order.size()));
+    AVX_CK(op->yf_coef.alloc(coef.size()));
+    AVX_CK(cudaMemcpy(op->yf_order.p, order.data(), order.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    AVX_CK(cudaMemcpy(op->yf_coef.p, coef.data(), coef.size() * sizeof(float2), cudaMemcpyHostToDevice));
+  } else if (op->tc_np) {
+    // coefficient tables of the tensor-core transforms (at most 48 rows per frame)
     std::vector<unsigned short> tab(avx::tc_ytab_bytes(H, T, np) / 2);
-    avx::tc_build_ytab(W, H, T, op->centered ? W / 2 : 0, op->centered ? H / 2 : 0, op->rows.data(),
-                       op->row_off.data(), np, tab.data());
+    avx::tc_build_ytab(W, H, T, op->centered ? W / 2 : 0, sy, op->rows.data(), op->row_off.data(), np, tab.data());
     AVX_CK(op->tc_ytab.alloc(tab.size() * 2 / sizeof(uint4)));
     AVX_CK(cudaMemcpy(op->tc_ytab.p, tab.data(), tab.size() * 2, cudaMemcpyHostToDevice));
     std::vector<unsigned short> ctab(avx::tc_ctab_bytes(H, T, np) / 2);
-    avx::tc_build_ctab(H, T, op->centered ? H / 2 : 0, op->rows.data(), op->row_off.data(), np, ctab.data());
+    avx::tc_build_ctab(H, T, sy, op->rows.data(), op->row_off.data(), np, ctab.data());
     AVX_CK(op->tc_ctab.alloc(ctab.size() * 2 / sizeof(uint4)));
     AVX_CK(cudaMemcpy(op->tc_ctab.p, ctab.data(), ctab.size() * 2, cudaMemcpyHostToDevice));
-    op->tc_np = np;
-    op->dft_mode = AVX_DFT_SPLIT_BF16X3;
   }
   return AVX_OK;
 }
@@ -637,7 +652,7 @@ struct avx_solver {
   bool own_stream = false;  // stream created by solver_alloc (else lent by the batch engine)
   // device state
   DevBuf<float2> prim, ext, dual, escr, z, d;
-  DevBuf<float2> b1t;  // coil maps in column-tile order (tensor-core adjoint)
+  DevBuf<float2> b1t;  // coil maps in the y-transforms' order (order_maps)
   DevBuf<DevState> st;
   DevBuf<double> pimg, pk, hist;
   int cap = 0;
@@ -891,8 +906,17 @@ static avx_status autotune(avx_solver* s, const float2* b1) {
   return AVX_OK;
 }
 
-static void set_tc(KArgs* k, const avx_operator* op) {
-  const bool on = op->kind == 0 && op->dft_mode == AVX_DFT_SPLIT_BF16X3 && op->tc_np > 0;
+// the split form runs on the tensor cores
+static bool uses_tc(const avx_operator* op) {
+  return op->kind == 0 && op->dft_mode == AVX_DFT_SPLIT_BF16X3 && op->tc_np > 0 && !op->yf_n1;
+}
+
+static void set_dft(KArgs* k, const avx_operator* op) {
+  k->yf_n1 = op->yf_n1;
+  k->yf_rows = op->max_rows;
+  k->yf_order = op->yf_order.p;
+  k->yf_coef = op->yf_coef.p;
+  const bool on = uses_tc(op);
   k->tc_ytab = on ? op->tc_ytab.p : nullptr;
   k->tc_np = on ? op->tc_np : 0;
   k->tc_ctab = on ? op->tc_ctab.p : nullptr;
@@ -913,18 +937,23 @@ static KArgs make_kargs(avx_solver* s, const float2* b1, const float2* in, const
   k.binary_mask = s->op->binary ? 1 : 0;
   k.st = s->st.p;
   k.partial = s->pk.p;
-  set_tc(&k, s->op);
+  set_dft(&k, s->op);
   k.b1t = s->b1t.p;
   k.rows_kc = s->rows_kc;
   k.rows_rt = s->rows_rt;
   return k;
 }
 
-// the tensor-core adjoint reads the coil maps in column-tile order
-static avx_status prepare_b1t(avx_solver* s, const float2* b1) {
-  if (s->op->kind != 0 || s->op->dft_mode != AVX_DFT_SPLIT_BF16X3 || s->op->tc_np == 0) return AVX_OK;
-  AVX_CK(s->b1t.alloc(avx::b1t_count(s->W, s->H, s->C)));
-  avx::launch_b1_tile_transpose(b1, s->b1t.p, s->W, s->H, s->C, s->stream);
+// the coil maps in the order the operator's y-transforms read them, into buf
+// (left alone when they read the maps as they are)
+static avx_status order_maps(const avx_operator* op, const float2* b1, DevBuf<float2>& buf, cudaStream_t s) {
+  if (op->yf_n1) {
+    AVX_CK(buf.alloc(avx::yfft_maps_count(op->W, op->H, op->C, op->yf_n1)));
+    avx::launch_yfft_maps(b1, buf.p, op->W, op->H, op->C, op->yf_n1, s);
+  } else if (uses_tc(op)) {
+    AVX_CK(buf.alloc(avx::b1t_count(op->W, op->H, op->C)));
+    avx::launch_b1_tile_transpose(b1, buf.p, op->W, op->H, op->C, s);
+  }
   AVX_CK(cudaGetLastError());
   return AVX_OK;
 }
@@ -1107,14 +1136,14 @@ static avx_status solver_begin(avx_solver* s, const float2* data, float2* x, con
   }
   r = prepare_run(s, data, x);
   if (r != AVX_OK) return r;
+  r = order_maps(s->op, b1, s->b1t, s->stream);
+  if (r != AVX_OK) return r;
   if (s->autotune && !s->tuned) {
     r = autotune(s, b1);
     if (r != AVX_OK) return r;
     r = prepare_run(s, data, x);  // the trial launches overwrote the fields
     if (r != AVX_OK) return r;
   }
-  r = prepare_b1t(s, b1);
-  if (r != AVX_OK) return r;
   if (s->method == AVX_METHOD_ICTGV2 && s->debug) {
     PDArgs a = make_pdargs(s);
     const KArgs kx = make_kargs(s, b1, s->primc(0), nullptr);
@@ -1770,8 +1799,13 @@ avx_status avx_operator_backward(avx_operator* op, const avx_cf32* d_x, avx_cf32
   k.in = reinterpret_cast<const float2*>(d_x);
   k.dense_out = reinterpret_cast<float2*>(d_k);
   k.qp = op->d_qp.p;  // y-transformed rows between the two kernels
-  set_tc(&k, op);
-  if (op->R) avx::launch_kspace(k, 3, 0);
+  set_dft(&k, op);
+  if (op->R) {
+    const avx_status r = order_maps(op, k.b1, op->b1t, 0);
+    if (r != AVX_OK) return r;
+    k.b1t = op->b1t.p;
+    avx::launch_kspace(k, 3, 0);
+  }
   AVX_CK(cudaGetLastError());
   AVX_CK(cudaDeviceSynchronize());
   return AVX_OK;
@@ -1792,12 +1826,10 @@ avx_status avx_operator_forward(avx_operator* op, avx_cf32* d_k, avx_cf32* d_x, 
   k.g = op->geom();
   k.b1 = reinterpret_cast<const float2*>(d_b1);
   k.qp = op->d_qp.p;
-  set_tc(&k, op);
-  if (k.tc_ctab) {
-    AVX_CK(op->tc_b1t.alloc(avx::b1t_count(op->W, op->H, op->C)));
-    avx::launch_b1_tile_transpose(k.b1, op->tc_b1t.p, op->W, op->H, op->C, 0);
-    k.b1t = op->tc_b1t.p;
-  }
+  set_dft(&k, op);
+  const avx_status r = order_maps(op, k.b1, op->b1t, 0);
+  if (r != AVX_OK) return r;
+  k.b1t = op->b1t.p;
   avx::launch_dense_rowidft(k.g, reinterpret_cast<float2*>(d_k), op->d_qp.p, op->has_mask ? op->d_mask.p : nullptr, 0);
   avx::launch_adjoint(k, reinterpret_cast<float2*>(d_x), 0);
   AVX_CK(cudaGetLastError());
@@ -1981,6 +2013,8 @@ avx_status avx_solver_adapt_step_size(avx_solver* s, const avx_cf32* const* d_di
     avx::launch_step_finalize(a, s->pimg.p, s->pk.p, avx::radial_interp_blocks(s->op->rg), s->p.sigmaTauRatio,
                               s->stream);
   } else {
+    r = order_maps(s->op, b1, s->b1t, s->stream);
+    if (r != AVX_OK) return r;
     const KArgs ke = make_kargs(s, b1, s->escrc(0), nullptr);
     avx::launch_step(s->method, a, ke, e, P, s->pimg.p, s->pk.p, s->p.sigmaTauRatio, s->stream);
   }
@@ -2003,7 +2037,7 @@ avx_status avx_solver_compute_gap(avx_solver* s, const avx_cf32* const* d_x, con
   const size_t N = (size_t)s->N();
   r = prepare_run(s, reinterpret_cast<const float2*>(d_data), nullptr);
   if (r != AVX_OK) return r;
-  r = prepare_b1t(s, reinterpret_cast<const float2*>(d_b1));
+  r = order_maps(s->op, reinterpret_cast<const float2*>(d_b1), s->b1t, s->stream);
   if (r != AVX_OK) return r;
   for (int c = 0; c < P; ++c)
     AVX_CK(cudaMemcpyAsync(s->primc(c), d_x[c], N * sizeof(float2), cudaMemcpyDeviceToDevice, s->stream));
@@ -2088,7 +2122,7 @@ static avx_status encoding_normal(avx_operator* op, const float2* b1, const floa
   k.in = u;
   k.qp = op->d_qp.p;
   k.st = st;
-  set_tc(&k, op);
+  set_dft(&k, op);
   k.b1t = b1t;
   avx::launch_kspace(k, 4, s);
   avx::launch_adjoint(k, img, s);
@@ -2167,10 +2201,10 @@ avx_status avx_operator_opnorm(avx_operator* op, const avx_cf32* d_x0, const avx
   if (iters < 1) return fail(AVX_E_ARG, "the power iteration needs at least one iteration");
   const float2* b1 = reinterpret_cast<const float2*>(d_b1);
   const float2* b1t = nullptr;
-  if (op->kind == 0 && op->dft_mode == AVX_DFT_SPLIT_BF16X3 && op->tc_np > 0) {
-    AVX_CK(op->tc_b1t.alloc(avx::b1t_count(op->W, op->H, op->C)));
-    avx::launch_b1_tile_transpose(b1, op->tc_b1t.p, op->W, op->H, op->C, 0);
-    b1t = op->tc_b1t.p;
+  {
+    const avx_status r = order_maps(op, b1, op->b1t, 0);
+    if (r != AVX_OK) return r;
+    b1t = op->b1t.p;
   }
   const Wts w0 = make_wts(1.f, 1.f, 1.f);
   return power_iteration(op, AVX_M_ENCODING, w0, w0, b1, b1t, reinterpret_cast<const float2*>(d_x0), iters, 0,
@@ -2186,7 +2220,7 @@ avx_status avx_solver_opnorm(avx_solver* s, const avx_cf32* d_x0, const avx_cf32
   r = solver_run_weights(s);
   if (r != AVX_OK) return r;
   const float2* b1 = reinterpret_cast<const float2*>(d_b1);
-  r = prepare_b1t(s, b1);
+  r = order_maps(s->op, b1, s->b1t, s->stream);
   if (r != AVX_OK) return r;
   Wts w1, w2;
   solver_weights(s, &w1, &w2);
@@ -2681,6 +2715,8 @@ size_t request_workspace(const avx_request& r, long long R_known, int max_rows_k
       b += avx::tc_ytab_bytes((int)H, (int)T, (int)np) + avx::tc_ctab_bytes((int)H, (int)T, (int)np);
       b += avx::b1t_count((int)W, (int)H, (int)C) * c8;
     }
+    if (const int n1 = max_rows > 0 ? avx::yfft_n1((int)H, (int)max_rows) : 0)
+      b += R * (8 + H / n1 * 8) + avx::yfft_maps_count((int)W, (int)H, (int)C, n1) * c8;
   } else {
     const size_t S = (size_t)r.n_fe * r.spokes_per_frame;
     const int isw = std::max(2, (int)r.sector_width);

@@ -67,7 +67,11 @@ struct KArgs {
   // split-BF16x3 tensor-core column adjoint (null: fp32 CUDA-core kernel)
   const uint4* tc_ctab; // conjugate coefficient pieces, tc_dft.cuh
   int tc_kc;            // MMA K (2 x rows per frame, rounded up to 16)
-  const float2* b1t;    // b1 in column-tile order for the tensor-core adjoint (tc_dft.cuh)
+  const float2* b1t;    // b1 in the order of the y-transforms in use (yfft.cuh, else tc_dft.cuh's adjoint)
+  // register-FFT y-transforms (yf_n1 = 0: not used), tables of yfft.cuh
+  int yf_n1, yf_rows;   // the FFT's length, the most sampled rows of a frame
+  const int2* yf_order;
+  const float2* yf_coef;
   // row-FFT schedule of the row kernel (chosen by the autotuner): compact rows
   // per pass (8, 12 or 16; 0 = 16) and the radix plan (0: the compile-time
   // plan of the length when there is one, 1: the run-time plan)

@@ -18,6 +18,7 @@
 #include "stencil.cuh"
 #include "fft.cuh"
 #include "tc_dft.cuh"
+#include "yfft.cuh"
 
 namespace avx {
 
@@ -1335,6 +1336,10 @@ void launch_primal(int method, const PDArgs& a, cudaStream_t s) {
 }
 
 void launch_ydft(const KArgs& k, cudaStream_t s) {
+  if (k.yf_n1) {
+    launch_yfft(k, s);
+    return;
+  }
   if (k.tc_ytab) {
     launch_ydft_tc(k, s);
     return;
@@ -1366,6 +1371,10 @@ void launch_kspace(const KArgs& k, int mode, cudaStream_t s) {
 }
 
 void launch_adjoint(const KArgs& k, float2* img, cudaStream_t s) {
+  if (k.yf_n1) {
+    launch_yfft_adjoint(k, img, s);
+    return;
+  }
   if (k.tc_ctab) {
     launch_coladj_tc(k, img, s);
     return;
