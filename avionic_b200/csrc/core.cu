@@ -36,6 +36,7 @@
 #include "radial.cuh"
 #include "tc_dft.cuh"
 #include "utils_kernels.cuh"
+#include "rowfft.cuh"
 #include "yfft.cuh"
 
 
@@ -266,6 +267,7 @@ avx_status configure_once() {
   AVX_CK(avx::configure_fft2d_kernels());
   AVX_CK(avx::configure_tc_kernels());
   AVX_CK(avx::configure_yfft_kernels());
+  AVX_CK(avx::configure_rowfft_kernels());
   g_configured |= bit;
   return AVX_OK;
 }
@@ -1830,7 +1832,9 @@ avx_status avx_operator_forward(avx_operator* op, avx_cf32* d_k, avx_cf32* d_x, 
   const avx_status r = order_maps(op, k.b1, op->b1t, 0);
   if (r != AVX_OK) return r;
   k.b1t = op->b1t.p;
-  avx::launch_dense_rowidft(k.g, reinterpret_cast<float2*>(d_k), op->d_qp.p, op->has_mask ? op->d_mask.p : nullptr, 0);
+  if (op->has_mask) avx::launch_mask_dense(k.g, reinterpret_cast<float2*>(d_k), op->d_mask.p, 0);
+  k.dense_in = reinterpret_cast<const float2*>(d_k);
+  if (op->R) avx::launch_rows(k, 5, 0);
   avx::launch_adjoint(k, reinterpret_cast<float2*>(d_x), 0);
   AVX_CK(cudaGetLastError());
   AVX_CK(cudaDeviceSynchronize());
@@ -2659,7 +2663,7 @@ avx_status avx_reconstruct_host(int method, unsigned W, unsigned H, unsigned C, 
   }
   // zero the data outside the mask (main.cpp:507-519): the compact rows only
   // read sampled rows, and the rest enter the gap's data term as zeros.
-  if (h_mask) avx::launch_dense_rowidft(pl.op->geom(), pl.dk.p, pl.op->d_qp.p, pl.dm.p, st);  // masks dk in place
+  if (h_mask) avx::launch_mask_dense(pl.op->geom(), pl.dk.p, pl.dm.p, st);
   AVX_CK(cudaGetLastError());
   r = avx_solver_run(pl.s, reinterpret_cast<avx_cf32*>(pl.dk.p), reinterpret_cast<avx_cf32*>(pl.dx.p),
                      reinterpret_cast<avx_cf32*>(pl.db1.p));

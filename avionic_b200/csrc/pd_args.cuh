@@ -57,6 +57,7 @@ struct KArgs {
   const float2* d;      // compact data
   float2* qp;           // compact row-inverse-transformed output
   float2* dense_out;    // dense k-space output (operator apply)
+  const float2* dense_in;  // dense k-space input (operator apply, adjoint)
   float lam;            // data weight lambda
   int binary_mask;      // 1 when every mask value is 0 or 1
   DevState* st;

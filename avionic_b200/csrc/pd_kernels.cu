@@ -18,6 +18,7 @@
 #include "stencil.cuh"
 #include "fft.cuh"
 #include "tc_dft.cuh"
+#include "rowfft.cuh"
 #include "yfft.cuh"
 
 namespace avx {
@@ -596,12 +597,14 @@ size_t ydft_smem_bytes(int H) { return sizeof(float2) * (size_t)H * (YD_XS + KSP
 //   1  step rule: sum |mask X|^2
 //   2  gap:       sum |mask X - d|^2, Re<d,z>, |z|^2, then z <- mask z and Q'
 //   3  apply:     dense_out[t,c,ky,kx] = mask X
+//   4  normal:    Q' of mask^2 X
+//   5  adjoint:   Q' of the sampled rows of the (masked) dense k-space dense_in
 // Each CTA reads and rewrites only its own block of k.qp.
 // ---------------------------------------------------------------------------
 
 template <int KC, int PLAN>
 __global__ void __launch_bounds__(256, 4) rows_kernel(KArgs a, int mode) {
-  if (a.st && a.st->stop && mode != 3) return;
+  if (a.st && a.st->stop && mode != 3 && mode != 5) return;
   constexpr int KCP = AVX_FFT_PITCH(KC);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const CartGeomDev& g = a.g;
@@ -640,7 +643,9 @@ __global__ void __launch_bounds__(256, 4) rows_kernel(KArgs a, int mode) {
       for (int b = 0; b < ROWS_RB; ++b) {
         const int e = e0 + b * nt;
         const int kk = fast_div(e, (unsigned)W, mW), x = e - kk * W;
-        v[b] = (e < KC * W && kk < kc) ? a.qp[zb + (long long)(k0 + kk) * W + x] : czero();
+        const float2* src = a.qp + zb + (long long)(k0 + kk) * W;
+        if (mode == 5 && kk < kc) src = a.dense_in + (((long long)t * C + c) * g.H + g.rows[r0 + k0 + kk]) * W;
+        v[b] = (e < KC * W && kk < kc) ? src[x] : czero();
       }
 #pragma unroll
       for (int b = 0; b < ROWS_RB; ++b) {
@@ -657,7 +662,9 @@ __global__ void __launch_bounds__(256, 4) rows_kernel(KArgs a, int mode) {
     }
     __syncthreads();
     float2* Xb = X;  // buffer holding the row transform, index (kx - sx) mod W with the FFT
-    if (g.nrad) {
+    if (mode == 5) {
+      Xb = P;
+    } else if (g.nrad) {
       Xb = row_fft_planned<KC, PLAN, +1>(P, X, twx, W, g.nrad, splan);
     } else {
       // dense DFT along x: thread per kx
@@ -684,7 +691,7 @@ __global__ void __launch_bounds__(256, 4) rows_kernel(KArgs a, int mode) {
     // pointwise stage on the kept samples; Xb[n] holds kx = n + sx (FFT) or kx.
     // The mask, z and d values of ROWS_RB samples are loaded first.
     const bool need_zd = mode == 0 || mode == 2;
-    for (int e0 = tid; e0 < kc * W; e0 += ROWS_RB * nt) {
+    for (int e0 = tid; e0 < kc * W && mode != 5; e0 += ROWS_RB * nt) {
       float mb[ROWS_RB];
       float2 zpre[ROWS_RB], dpre[ROWS_RB];
 #pragma unroll
@@ -767,7 +774,7 @@ __global__ void __launch_bounds__(256, 4) rows_kernel(KArgs a, int mode) {
       for (int kx = 0; kx < W; ++kx) {
         const float2 tw = twx[jj];
         const float2 twc = make_float2(tw.x, -tw.y);
-        const float2* xr = X + kx * KCP;
+        const float2* xr = Xb + kx * KCP;
 #pragma unroll
         for (int kk = 0; kk < KC; ++kk) cfma(acc[kk], twc, xr[kk]);
         jj += step;
@@ -1214,36 +1221,19 @@ __global__ void gather_rows_kernel(CartGeomDev g, const float2* dense, float2* c
 
 // k-space -> image transform of a dense k-space vector, first stage: mask the
 // input in place (cartesian_operator.cpp:83-88; rows outside the kept set
-// carry mask 0 and are cleared) and row-IDFT the kept rows into Q'.
-__global__ void dense_rowidft_kernel(CartGeomDev g, float2* dense, float2* qp, const float* mask_dense) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* row = reinterpret_cast<float2*>(smem_raw);  // [W]
-  const int c = blockIdx.x % g.C, t = blockIdx.x / g.C;
-  const int r0 = g.row_off[t], r1 = g.row_off[t + 1];
-  const long long zb = kbase(g, t, c, r0, r1);
-  float2* slice = dense + ((long long)t * g.C + c) * g.H * g.W;
-  if (mask_dense) {
-    const float* ms = mask_dense + (long long)t * g.H * g.W;
-    for (long long e = threadIdx.x; e < (long long)g.H * g.W; e += blockDim.x) slice[e] = cscale(slice[e], ms[e]);
-  }
-  __syncthreads();
-  for (int kk = 0; kk < r1 - r0; ++kk) {
-    const int ky = g.rows[r0 + kk];
-    for (int kx = threadIdx.x; kx < g.W; kx += blockDim.x) row[kx] = slice[(long long)ky * g.W + kx];
-    __syncthreads();
-    for (int x = threadIdx.x; x < g.W; x += blockDim.x) {
-      float2 acc = czero();
-      const int step = (x - g.sx + g.W) % g.W;
-      int jj = (step * ((g.W - g.sx) % g.W)) % g.W;
-      for (int kx = 0; kx < g.W; ++kx) {
-        const float2 tw = g.twx[jj];
-        cfma(acc, make_float2(tw.x, -tw.y), row[kx]);
-        jj += step;
-        if (jj >= g.W) jj -= g.W;
-      }
-      qp[zb + (long long)kk * g.W + x] = cscale(acc, g.inv_sqrt_w);
-    }
-    __syncthreads();
+// carry mask 0 and are cleared).  Values that the mask leaves as they are
+// (a mask of 1, zeros already cleared) are not stored: data that arrives
+// masked, as a solver's does, costs its read alone.
+__global__ void mask_dense_kernel(float2* dense, const float* __restrict__ mask, long long HW, int C) {
+  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (e >= HW) return;
+  const int t = blockIdx.y;
+  const float m = mask[t * HW + e];
+  float2* d = dense + (long long)t * C * HW + e;
+#pragma unroll 4
+  for (int c = 0; c < C; ++c) {
+    const float2 v = d[c * HW], w = cscale(v, m);
+    if (__float_as_uint(v.x) != __float_as_uint(w.x) || __float_as_uint(v.y) != __float_as_uint(w.y)) d[c * HW] = w;
   }
 }
 
@@ -1358,6 +1348,11 @@ static void launch_rows_kc(const KArgs& k, int mode, cudaStream_t s) {
 }
 
 void launch_rows(const KArgs& k, int mode, cudaStream_t s) {
+  int n1, n2;
+  if (!k.rows_rt && rowfft_split(k.g.W, &n1, &n2)) {
+    launch_rowfft(k, mode, s);
+    return;
+  }
   switch (k.rows_kc) {
     case 8: launch_rows_kc<8>(k, mode, s); break;
     case 12: launch_rows_kc<12>(k, mode, s); break;
@@ -1458,8 +1453,9 @@ void launch_gather_rows(const CartGeomDev& g, const float2* dense, float2* compa
   gather_rows_kernel<<<g.C * g.T, 256, 0, s>>>(g, dense, compact, apply_mask);
 }
 
-void launch_dense_rowidft(const CartGeomDev& g, float2* dense, float2* qp, const float* mask_dense, cudaStream_t s) {
-  dense_rowidft_kernel<<<g.C * g.T, 256, sizeof(float2) * g.W, s>>>(g, dense, qp, mask_dense);
+void launch_mask_dense(const CartGeomDev& g, float2* dense, const float* mask, cudaStream_t s) {
+  const long long HW = (long long)g.W * g.H;
+  mask_dense_kernel<<<dim3((unsigned)((HW + 255) / 256), g.T), 256, 0, s>>>(dense, mask, HW, g.C);
 }
 
 cudaError_t configure_kernels() {

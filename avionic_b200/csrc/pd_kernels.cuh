@@ -60,7 +60,8 @@ void launch_gap_tail(int method, const PDArgs& a, const KArgs& k_x, double* pimg
                      const GapConst& gc, double* hg, double* hn, double* hf, int cap, int init_only,
                      cudaStream_t s);
 // y-transform followed by the row kernel in the given mode (0 PD step, 1 step-rule norm, 2 gap, 3 apply,
-// 4 normal operator: Q' = row-IFFT(mask^2 X), for A^H A by the column adjoint)
+// 4 normal operator: Q' = row-IFFT(mask^2 X), for A^H A by the column adjoint); launch_rows' mode 5 takes the
+// sampled rows of k.dense_in instead of the y-transform: Q' = row-IFFT of them
 void launch_kspace(const KArgs& k, int mode, cudaStream_t s);
 // img[t] = sum_c conj(b1_c) column-IDFT of the compact rows in k.qp
 void launch_adjoint(const KArgs& k, float2* img, cudaStream_t s);
@@ -70,7 +71,7 @@ void launch_gap(int method, const PDArgs& a, const KArgs& k_x, float2* khz, doub
                 const GapConst& gc, double* hg, double* hn, double* hf, int cap, int init_only, cudaStream_t s);
 void launch_gather_rows(const CartGeomDev& g, const float2* dense, float2* compact, int apply_mask,
                         cudaStream_t s);
-void launch_dense_rowidft(const CartGeomDev& g, float2* dense, float2* qp, const float* mask_dense,
-                          cudaStream_t s);
+// dense *= mask (T x H x W), in place
+void launch_mask_dense(const CartGeomDev& g, float2* dense, const float* mask, cudaStream_t s);
 
 }  // namespace avx

@@ -1,0 +1,17 @@
+// Row transforms of the Cartesian operator with two-step register FFTs (rowfft.cu).
+#pragma once
+
+#include "pd_args.cuh"
+
+namespace avx {
+
+// W = n1 n2 with 8 <= n2 <= n1 <= 16, or n1 = 20; false when W has no such split
+bool rowfft_split(int W, int* n1, int* n2);
+
+// the row kernel's work (launch_rows of pd_kernels.cuh) for a length with a
+// split; mode 5: Q' = row-IFFT of the sampled rows of the dense k-space in
+// k.dense_in (already masked)
+void launch_rowfft(const KArgs& k, int mode, cudaStream_t s);
+cudaError_t configure_rowfft_kernels();
+
+}  // namespace avx

@@ -1,0 +1,57 @@
+// Row FFT instances (rowfft_impl.cuh), first step of 8 to 12 points, and the dispatch.
+#include "rowfft_impl.cuh"
+
+namespace avx {
+
+ROWFFT_DEFINE(8)
+ROWFFT_DEFINE(9)
+ROWFFT_DEFINE(10)
+ROWFFT_DEFINE(11)
+ROWFFT_DEFINE(12)
+
+bool rowfft_split(int W, int* n1, int* n2) {
+  // the most balanced split: the fewest threads of a row idle in either step
+  for (int a : {8, 9, 10, 11, 12, 13, 14, 15, 16, 20}) {
+    if (W % a) continue;
+    const int b = W / a;
+    if (b < 8 || b > a || b > 16) continue;
+    *n1 = a;
+    *n2 = b;
+    return true;
+  }
+  return false;
+}
+
+void launch_rowfft(const KArgs& k, int mode, cudaStream_t s) {
+  int n1 = 0, n2 = 0;
+  if (!rowfft_split(k.g.W, &n1, &n2)) return;
+#define CALL_W(N) \
+  case N: rowfft_launch_##N(n2, k, mode, s); break;
+  switch (n1) {
+    CALL_W(8)
+    CALL_W(9)
+    CALL_W(10)
+    CALL_W(11)
+    CALL_W(12)
+    CALL_W(13)
+    CALL_W(14)
+    CALL_W(15)
+    CALL_W(16)
+    CALL_W(20)
+    default: break;
+  }
+#undef CALL_W
+}
+
+cudaError_t configure_rowfft_kernels() {
+  cudaError_t (*const all[])() = {rowfft_configure_8,  rowfft_configure_9,  rowfft_configure_10, rowfft_configure_11,
+                                  rowfft_configure_12, rowfft_configure_13, rowfft_configure_14, rowfft_configure_15,
+                                  rowfft_configure_16, rowfft_configure_20};
+  for (auto f : all) {
+    const cudaError_t e = f();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace avx

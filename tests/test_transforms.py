@@ -63,3 +63,43 @@ def test_y_transform_matches_oracle(H, rows, C, centered):
 @pytest.mark.parametrize("H,rows", [(34, 7), (37, 20), (4 * 29, 30)])
 def test_heights_without_a_register_fft(H, rows, dft):
     _check(24, H, 3, 3, rows, True, REL_DENSE, dft)
+
+
+# two-step row FFTs: the shortest and longest of each first length, odd widths (8-byte row copies), row counts
+# around the rows of a pass; 22, 62 and 251 have none (rows_kernel, dense)
+X_CASES = [(64, 5), (99, 17), (100, 16), (121, 1), (144, 12), (143, 8), (196, 24), (225, 33), (128, 9), (256, 7),
+           (160, 40), (320, 13), (22, 6), (62, 5), (251, 3)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("centered", [False, True])
+@pytest.mark.parametrize("W,rows", X_CASES)
+def test_row_transform_matches_oracle(W, rows, centered):
+    _check(W, 48, 3, 3, rows, centered, REL_DENSE if W in (62, 251) else REL_FFT)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,centered", [(64, False), (99, True), (160, True), (22, False)])
+def test_reconstruction_through_the_row_transform(W, centered):
+    """The z update inside the row kernel, with a weighted mask: 30 TV iterations against the oracle (fp32
+    iterates stay within a few 1e-6 of float64 this early; 1e-5)."""
+    import torch
+
+    import avionic_b200 as av
+    from avionic_b200 import synth
+    from oracle import solvers as so
+    prob = synth.small(W, H=40, W=W, T=3, C=3, binary=False)
+    T, C, H, _ = prob["kdata"].shape
+    op = av.CartesianOperator(W, H, C, T, mask=av.to_device(prob["mask"]), centered=centered)
+    s = av.Solver("TV", op)
+    p = s.params
+    p.maxIt = 30
+    s.params = p
+    x = torch.zeros((T, H, W), dtype=torch.complex64, device="cuda")
+    s.run(av.to_device(prob["kdata"]), x, av.to_device(prob["b1"]))
+    oop = OCart(W, H, C, T, mask=prob["mask"], centered=centered)
+    q = so.init_params("TV")
+    q.lam = oop.adapt_lambda(*q.adapt_kd)
+    q.maxIt = 30
+    xo = so.tv(prob["kdata"].astype(complex), np.zeros((T, H, W), complex), prob["b1"].astype(complex), oop, q)
+    assert _rel(x.cpu().numpy(), xo) < 1e-5
