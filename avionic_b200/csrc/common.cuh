@@ -73,6 +73,34 @@ struct DevState {
   double gap0;            // first normalised gap of the run (relative stop criterion)
 };
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may
+// start while its predecessor still runs.  Until pdl_wait() it reads only what
+// no kernel writes (an operator's tables); pdl_wait() returns once the
+// predecessor has completed and its writes are visible, and as every kernel of
+// a chain waits, once everything before it has too.  pdl_trigger() lets the
+// successor start once every CTA of this kernel has called it (or ended).  It
+// follows pdl_wait(), so that one kernel at most waits on the SMs ahead of its
+// turn: triggered at their start, whole chains of waiting CTAs kept the dual
+// update beside them off the SMs (294 x 24, 4 coils: 50 us an iteration
+// against 32).
+AVX_D void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+AVX_D void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Number of FP64 partial-sum slots a reduction writes per block.
 #define AVX_RED_SLOTS 12
 #define AVX_RED_BLOCKS 592  // 4 x 148 SMs

@@ -637,6 +637,10 @@ static HostPlan g_plan;
 // Solver
 // ===========================================================================
 
+// plain iterations per graph launch where that many follow one another (49 lie between two step rules)
+constexpr unsigned kChunk = 7;
+constexpr int kChunkShape = 4;
+
 struct avx_solver {
   int method = 0;
   int W = 0, H = 0, C = 0, T = 0;
@@ -661,8 +665,12 @@ struct avx_solver {
   double d_off_energy = 0.0;
   avx_run_stats stats{};
   DevState last{};
-  // graphs of the four iteration shapes
-  cudaGraphExec_t gexec[4] = {nullptr, nullptr, nullptr, nullptr};
+  // graphs of the four iteration shapes, and of kChunk plain iterations in a row
+  cudaGraphExec_t gexec[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  // streams the graphs are captured on, whose priorities their kernels take:
+  // the k-space stages and the primal update before the dual update beside them
+  cudaStream_t capture = nullptr;
+  avx::SideStream side;
   size_t graph_key = 0;
   // timing mode
   bool timing = false;
@@ -674,6 +682,9 @@ struct avx_solver {
     drop_graphs();
     for (auto e : events) cudaEventDestroy(e);
     if (stream && own_stream) cudaStreamDestroy(stream);
+    if (side.ev) cudaEventDestroy(side.ev);
+    if (side.side) cudaStreamDestroy(side.side);
+    if (capture) cudaStreamDestroy(capture);
   }
   void drop_graphs() {
     for (auto& g : gexec)
@@ -812,7 +823,6 @@ static avx_status tune_rows(avx_solver* s, const float2* b1) {
   const bool has_fixed = fft_plan_id(g.W, g.nrad, g.rad) != fft_plan_id_runtime(g.nrad, g.rad);
   const int cand[4][2] = {{KSPACE_KC, 0}, {12, 0}, {8, 0}, {KSPACE_KC, 1}};
   const int ncand = has_fixed ? 4 : 3;
-  avx::launch_ydft(k, s->stream);  // compact rows for the trial launches to transform
   cudaEvent_t e0, e1;
   AVX_CK(cudaEventCreate(&e0));
   AVX_CK(cudaEventCreate(&e1));
@@ -820,9 +830,16 @@ static avx_status tune_rows(avx_solver* s, const float2* b1) {
   for (int i = 0; i < ncand; ++i) {
     k.rows_kc = cand[i][0];
     k.rows_rt = cand[i][1];
-    for (int w = 0; w < 3; ++w) avx::launch_rows(k, 0, s->stream);
+    // between its neighbours of an iteration: launches of the row kernel alone overlap one another, which
+    // favours small passes (cine: 8 rows a pass tie with 16 alone, but cost 7 us of an iteration)
+    auto chain = [&] {
+      avx::launch_ydft(k, s->stream);
+      avx::launch_rows(k, 0, s->stream);
+      avx::launch_adjoint(k, s->op->r_khz.p, s->stream);
+    };
+    for (int w = 0; w < 2; ++w) chain();
     cudaEventRecord(e0, s->stream);
-    for (int w = 0; w < 5; ++w) avx::launch_rows(k, 0, s->stream);
+    for (int w = 0; w < 5; ++w) chain();
     cudaEventRecord(e1, s->stream);
     cudaError_t ce = cudaEventSynchronize(e1);
     float ms = 0.f;
@@ -1012,13 +1029,16 @@ static void radial_pass(avx_solver* s, int mode, const float2* b1, const float2*
   if (ev) cudaEventRecord(ev[2], s->stream);
 }
 
-static void enqueue_shape_radial(avx_solver* s, int shape, const float2* b1, cudaEvent_t* ev) {
+static void enqueue_shape_radial(avx_solver* s, int shape, const float2* b1, const avx::SideStream& side,
+                                 cudaEvent_t* ev) {
   const PDArgs a = make_pdargs(s);
   const KArgs kdummy = make_kargs(s, b1, s->extc(0), nullptr);
   if (ev) cudaEventRecord(ev[0], s->stream);
-  avx::launch_dual(s->method, a, s->stream);
+  side.fork(s->stream);
+  avx::launch_dual(s->method, a, side.side ? side.side : s->stream);
   if (ev) cudaEventRecord(ev[1], s->stream);
   radial_pass(s, 0, b1, s->extc(0), nullptr, ev ? ev + 2 : nullptr);
+  side.join(s->stream);
   avx::launch_primal(s->method, a, s->stream);
   if (ev) cudaEventRecord(ev[5], s->stream);
   const int nk = avx::radial_interp_blocks(s->op->rg);
@@ -1039,14 +1059,15 @@ static void enqueue_shape_radial(avx_solver* s, int shape, const float2* b1, cud
   }
 }
 
-static void enqueue_shape(avx_solver* s, int shape, const float2* b1, cudaEvent_t* ev = nullptr) {
+static void enqueue_shape(avx_solver* s, int shape, const float2* b1, const avx::SideStream& side,
+                          cudaEvent_t* ev = nullptr) {
   if (s->op->kind == 1) {
-    enqueue_shape_radial(s, shape, b1, ev);
+    enqueue_shape_radial(s, shape, b1, side, ev);
     return;
   }
   const PDArgs a = make_pdargs(s);
   const KArgs ks = make_kargs(s, b1, s->extc(0), nullptr);
-  avx::launch_iteration(s->method, a, ks, s->op->r_khz.p, s->stream, ev);
+  avx::launch_iteration(s->method, a, ks, s->op->r_khz.p, s->stream, side, ev);
   if (shape & 1) {
     avx::Ptr8 e;
     const int P = method_P(s->method);
@@ -1176,14 +1197,28 @@ static avx_status solver_begin(avx_solver* s, const float2* data, float2* x, con
   return AVX_OK;
 }
 
-// The CUDA graph of iteration shape `shape` (bit 0: step rule, bit 1: gap),
-// captured on the solver's stream at first use.
+// The CUDA graph of iteration shape `shape` (bit 0: step rule, bit 1: gap;
+// kChunkShape: kChunk plain iterations), captured at first use on a stream of
+// the solver's own.
 static avx_status solver_graph(avx_solver* s, int shape, const float2* b1) {
   if (s->gexec[shape]) return AVX_OK;
+  if (!s->capture) {
+    int least = 0, greatest = 0;
+    AVX_CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    AVX_CK(cudaStreamCreateWithPriority(&s->capture, cudaStreamNonBlocking, greatest));
+    AVX_CK(cudaStreamCreateWithPriority(&s->side.side, cudaStreamNonBlocking, least));
+    AVX_CK(cudaEventCreateWithFlags(&s->side.ev, cudaEventDisableTiming));
+  }
   cudaGraph_t g;
-  AVX_CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-  enqueue_shape(s, shape, b1);
-  AVX_CK(cudaStreamEndCapture(s->stream, &g));
+  AVX_CK(cudaStreamBeginCapture(s->capture, cudaStreamCaptureModeThreadLocal));
+  const cudaStream_t run = s->stream;
+  s->stream = s->capture;  // the launches below go to the capture
+  if (shape == kChunkShape)
+    for (unsigned i = 0; i < kChunk; ++i) enqueue_shape(s, 0, b1, s->side);
+  else
+    enqueue_shape(s, shape, b1, s->side);
+  s->stream = run;
+  AVX_CK(cudaStreamEndCapture(s->capture, &g));
   const cudaError_t e = cudaGraphInstantiate(&s->gexec[shape], g, 0);
   cudaGraphDestroy(g);
   AVX_CK(e);
@@ -1192,15 +1227,25 @@ static avx_status solver_graph(avx_solver* s, int shape, const float2* b1) {
 
 static int iter_shape(const avx_solver* s, unsigned k) { return (step_due(k) ? 1 : 0) | (gap_due(s, k) ? 2 : 0); }
 
+// The graph that iterations k, k + 1, ... < k1 start with, and how many of them it runs.
+static int next_graph(const avx_solver* s, unsigned k, unsigned k1, unsigned* n) {
+  *n = 1;
+  if (k + kChunk > k1) return iter_shape(s, k);
+  for (unsigned i = 0; i < kChunk; ++i)
+    if (iter_shape(s, k + i)) return iter_shape(s, k);
+  *n = kChunk;
+  return kChunkShape;
+}
+
 // Enqueues iterations [k0, k1) from the graphs of their shapes (no host
 // synchronisation); *launches receives the kernels they hold.
 static avx_status solver_enqueue(avx_solver* s, const float2* b1, unsigned k0, unsigned k1, unsigned* launches) {
-  for (unsigned k = k0; k < k1; ++k) {
-    const int shape = iter_shape(s, k);
+  for (unsigned k = k0, n; k < k1; k += n) {
+    const int shape = next_graph(s, k, k1, &n);
     avx_status r = solver_graph(s, shape, b1);
     if (r != AVX_OK) return r;
     AVX_CK(cudaGraphLaunch(s->gexec[shape], s->stream));
-    if (launches) *launches += shape_launches(s->op->kind, shape);
+    if (launches) *launches += n * shape_launches(s->op->kind, shape == kChunkShape ? 0 : shape);
   }
   return AVX_OK;
 }
@@ -1239,24 +1284,25 @@ static avx_status solver_run(avx_solver* s, const float2* data, float2* x, const
   unsigned launches = 0;
   AVX_CK(cudaEventRecord(ev0, s->stream));
   unsigned k = 0;
-  for (; k < s->p.maxIt; ++k) {
-    const int shape = iter_shape(s, k);
+  while (k < s->p.maxIt) {
     if (s->timing) {
+      const int shape = iter_shape(s, k);
       launches += shape_launches(s->op->kind, shape);
-      enqueue_shape(s, shape, b1, &s->events[NEV * k]);
+      enqueue_shape(s, shape, b1, avx::SideStream(), &s->events[NEV * k]);
       AVX_CK(cudaGetLastError());
+      ++k;
       continue;
     }
-    r = solver_enqueue(s, b1, k, k + 1, &launches);
+    // to the end, or with a stop test through the next iteration whose gap the host looks at (k % 100 == 0)
+    const unsigned k1 = stop_active(s) ? std::min(s->p.maxIt, (k + 99) / 100 * 100 + 1) : s->p.maxIt;
+    r = solver_enqueue(s, b1, k, k1, &launches);
     if (r != AVX_OK) return r;
-    if (stop_active(s) && (shape & 2) && (k % 100 == 0)) {
+    k = k1;
+    if (stop_active(s) && (iter_shape(s, k - 1) & 2) && ((k - 1) % 100 == 0)) {
       int stop = 0;
       AVX_CK(cudaMemcpyAsync(&stop, &s->st.p->stop, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
       AVX_CK(cudaStreamSynchronize(s->stream));
-      if (stop) {
-        ++k;
-        break;
-      }
+      if (stop) break;
     }
   }
   AVX_CK(cudaEventRecord(ev1, s->stream));
@@ -2787,8 +2833,9 @@ avx_status job_setup(Job* j) {
     e = solver_begin(j->s, reinterpret_cast<const float2*>(r.d_data), reinterpret_cast<float2*>(r.d_x),
                      reinterpret_cast<const float2*>(r.d_b1));
   // the graphs of every iteration shape the run takes
-  for (unsigned k = 0; e == AVX_OK && k < j->s->p.maxIt; ++k) e = solver_graph(j->s, iter_shape(j->s, k),
-                                                                                reinterpret_cast<const float2*>(r.d_b1));
+  for (unsigned k = 0, n; e == AVX_OK && k < j->s->p.maxIt; k += n)
+    e = solver_graph(j->s, next_graph(j->s, k, std::min(j->s->p.maxIt, (k / kSlice + 1) * kSlice), &n),
+                     reinterpret_cast<const float2*>(r.d_b1));
   if (e == AVX_OK) {
     const cudaError_t ce = cudaStreamSynchronize(j->stream);
     if (ce != cudaSuccess) e = fail(AVX_E_CUDA, std::string("request set-up: ") + cudaGetErrorString(ce));

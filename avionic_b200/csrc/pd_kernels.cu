@@ -29,6 +29,8 @@ namespace avx {
 
 template <int M, int NT>
 __global__ void __launch_bounds__(NT) dual_kernel(PDArgs a) {
+  pdl_wait();
+  pdl_trigger();
   if (a.st->stop) return;
   // iteration counter (loopCnt of the reference) kept on the device so that
   // every iteration launches identical work and can be replayed from a graph
@@ -220,6 +222,8 @@ AVX_D float2 bt(const Nb& n, int k, int t, int T) {
 
 template <int M, int NT>
 __global__ void __launch_bounds__(NT) dual_vec_kernel(PDArgs a) {
+  pdl_wait();
+  pdl_trigger();
   if (a.st->stop) return;
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.st->iters += 1;
   const int HW2 = (a.W >> 1) * a.H;
@@ -428,6 +432,8 @@ AVX_D void pair_symdiv(const DivBranch& b, int k, int x, int y, int t, int W, in
 // divergence, which is all that crosses the phases.
 template <int M, int NT>
 __global__ void __launch_bounds__(NT) primal_vec_kernel(PDArgs a) {
+  pdl_wait();
+  pdl_trigger();
   if (a.st->stop) return;
   const int HW2 = (a.W >> 1) * a.H;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -892,6 +898,8 @@ __global__ void __launch_bounds__(CA_TX* CA_TY) coladj_kernel(KArgs k, float2* i
 
 template <int M, int PR_TX, int PR_TY, int PR_YP>
 __global__ void __launch_bounds__(PR_TX* PR_TY) primal_kernel(PDArgs a) {
+  pdl_wait();
+  pdl_trigger();
   if (a.st->stop) return;
   constexpr int PR_TH = PR_TY * PR_YP;
   const int t = blockIdx.z;
@@ -1258,11 +1266,11 @@ int dual_block_threads(int i) { return kDualBlocks[(i >= 0 && i < AVX_DUAL_BLOCK
 template <int NT>
 static void launch_dual_nt(int method, const PDArgs& a, cudaStream_t s) {
   dim3 gd((a.W * a.H + NT - 1) / NT, a.T);
-  if (method == AVX_M_TV) dual_kernel<AVX_M_TV, NT><<<gd, NT, 0, s>>>(a);
-  else if (method == AVX_M_TVTEMP) dual_kernel<AVX_M_TVTEMP, NT><<<gd, NT, 0, s>>>(a);
-  else if (method == AVX_M_TGV2) dual_kernel<AVX_M_TGV2, NT><<<gd, NT, 0, s>>>(a);
-  else if (method == AVX_M_ICTV) dual_kernel<AVX_M_ICTV, NT><<<gd, NT, 0, s>>>(a);
-  else dual_kernel<AVX_M_ICTGV2, NT><<<gd, NT, 0, s>>>(a);
+  if (method == AVX_M_TV) launch_dependent(dual_kernel<AVX_M_TV, NT>, gd, NT, 0, s, a);
+  else if (method == AVX_M_TVTEMP) launch_dependent(dual_kernel<AVX_M_TVTEMP, NT>, gd, NT, 0, s, a);
+  else if (method == AVX_M_TGV2) launch_dependent(dual_kernel<AVX_M_TGV2, NT>, gd, NT, 0, s, a);
+  else if (method == AVX_M_ICTV) launch_dependent(dual_kernel<AVX_M_ICTV, NT>, gd, NT, 0, s, a);
+  else launch_dependent(dual_kernel<AVX_M_ICTGV2, NT>, gd, NT, 0, s, a);
 }
 
 bool dual_pairs(int method, int W) { return (method == AVX_M_TGV2 || method == AVX_M_ICTGV2) && W % 2 == 0; }
@@ -1270,8 +1278,8 @@ bool dual_pairs(int method, int W) { return (method == AVX_M_TGV2 || method == A
 template <int NT>
 static void launch_dual_vec(int method, const PDArgs& a, cudaStream_t s) {
   dim3 gd(((a.W / 2) * a.H + NT - 1) / NT, a.T);
-  if (method == AVX_M_TGV2) dual_vec_kernel<AVX_M_TGV2, NT><<<gd, NT, 0, s>>>(a);
-  else dual_vec_kernel<AVX_M_ICTGV2, NT><<<gd, NT, 0, s>>>(a);
+  if (method == AVX_M_TGV2) launch_dependent(dual_vec_kernel<AVX_M_TGV2, NT>, gd, NT, 0, s, a);
+  else launch_dependent(dual_vec_kernel<AVX_M_ICTGV2, NT>, gd, NT, 0, s, a);
 }
 
 void launch_dual(int method, const PDArgs& a, cudaStream_t s) {
@@ -1294,18 +1302,18 @@ template <int TX, int TY, int YP>
 static void launch_primal_tile(int method, const PDArgs& a, cudaStream_t s) {
   dim3 gp((a.W + TX - 1) / TX, (a.H + TY * YP - 1) / (TY * YP), a.T);
   dim3 bl(TX, TY);
-  if (method == AVX_M_TV) primal_kernel<AVX_M_TV, TX, TY, YP><<<gp, bl, 0, s>>>(a);
-  else if (method == AVX_M_TVTEMP) primal_kernel<AVX_M_TVTEMP, TX, TY, YP><<<gp, bl, 0, s>>>(a);
-  else if (method == AVX_M_TGV2) primal_kernel<AVX_M_TGV2, TX, TY, YP><<<gp, bl, 0, s>>>(a);
-  else if (method == AVX_M_ICTV) primal_kernel<AVX_M_ICTV, TX, TY, YP><<<gp, bl, 0, s>>>(a);
-  else primal_kernel<AVX_M_ICTGV2, TX, TY, YP><<<gp, bl, 0, s>>>(a);
+  if (method == AVX_M_TV) launch_dependent(primal_kernel<AVX_M_TV, TX, TY, YP>, gp, bl, 0, s, a);
+  else if (method == AVX_M_TVTEMP) launch_dependent(primal_kernel<AVX_M_TVTEMP, TX, TY, YP>, gp, bl, 0, s, a);
+  else if (method == AVX_M_TGV2) launch_dependent(primal_kernel<AVX_M_TGV2, TX, TY, YP>, gp, bl, 0, s, a);
+  else if (method == AVX_M_ICTV) launch_dependent(primal_kernel<AVX_M_ICTV, TX, TY, YP>, gp, bl, 0, s, a);
+  else launch_dependent(primal_kernel<AVX_M_ICTGV2, TX, TY, YP>, gp, bl, 0, s, a);
 }
 
 template <int NT>
 static void launch_primal_vec(int method, const PDArgs& a, cudaStream_t s) {
   dim3 gd(((a.W / 2) * a.H + NT - 1) / NT, a.T);
-  if (method == AVX_M_TGV2) primal_vec_kernel<AVX_M_TGV2, NT><<<gd, NT, 0, s>>>(a);
-  else primal_vec_kernel<AVX_M_ICTGV2, NT><<<gd, NT, 0, s>>>(a);
+  if (method == AVX_M_TGV2) launch_dependent(primal_vec_kernel<AVX_M_TGV2, NT>, gd, NT, 0, s, a);
+  else launch_dependent(primal_vec_kernel<AVX_M_ICTGV2, NT>, gd, NT, 0, s, a);
 }
 
 void launch_primal(int method, const PDArgs& a, cudaStream_t s) {
@@ -1342,6 +1350,8 @@ template <int KC>
 static void launch_rows_kc(const KArgs& k, int mode, cudaStream_t s) {
   // 256 threads, as the compile-time FFT plans assume
   const int id = k.rows_rt ? fft_plan_id_runtime(k.g.nrad, k.g.rad) : fft_plan_id(k.g.W, k.g.nrad, k.g.rad);
+  // launched in plain stream order: as a dependent launch its CTAs, resident early with up to 100 KB of shared
+  // memory each, hold up what runs beside them (294 x 24, 4 coils: 50 us an iteration against 31)
 #define CALL_R(ID) rows_kernel<KC, ID><<<k.g.C * k.g.T, 256, rows_smem_bytes(k.g.W, KC), s>>>(k, mode)
   AVX_FFT_PLAN_DISPATCH(id, CALL_R)
 #undef CALL_R
@@ -1378,9 +1388,28 @@ void launch_adjoint(const KArgs& k, float2* img, cudaStream_t s) {
   coladj_kernel<<<gr, dim3(CA_TX, CA_TY), 0, s>>>(k, img);
 }
 
-void launch_iteration(int method, const PDArgs& a, const KArgs& k, float2* khz, cudaStream_t s, cudaEvent_t* ev) {
+void SideStream::fork(cudaStream_t main) const {
+  if (!side) return;
+  cudaEventRecord(ev, main);
+  cudaStreamWaitEvent(side, ev, 0);
+}
+void SideStream::join(cudaStream_t main) const {
+  if (!side) return;
+  cudaEventRecord(ev, side);
+  cudaStreamWaitEvent(main, ev, 0);
+}
+
+void launch_iteration(int method, const PDArgs& a, const KArgs& k, float2* khz, cudaStream_t s,
+                      const SideStream& side, cudaEvent_t* ev) {
+  // Beside the dense fp32 sums or the Stockham row kernel (large shared-memory tiles, which leave the dual
+  // update's stencil little L1) the two only lengthen one another: 84 x 101, 35 frames, 10 coils, 50 rows 308 us
+  // an iteration with the dual update beside them, 296 before them; 251 x 174, 46 frames, 4 coils 398 and 327.
+  int n1, n2;
+  const SideStream beside =
+      (k.yf_n1 || k.tc_ytab) && !k.rows_rt && rowfft_split(k.g.W, &n1, &n2) ? side : SideStream();
   rec(ev, 0, s);
-  launch_dual(method, a, s);
+  beside.fork(s);
+  launch_dual(method, a, beside.side ? beside.side : s);
   rec(ev, 1, s);
   launch_ydft(k, s);
   rec(ev, 2, s);
@@ -1388,6 +1417,7 @@ void launch_iteration(int method, const PDArgs& a, const KArgs& k, float2* khz, 
   rec(ev, 3, s);
   launch_adjoint(k, khz, s);
   rec(ev, 4, s);
+  beside.join(s);
   launch_primal(method, a, s);
   rec(ev, 5, s);
 }

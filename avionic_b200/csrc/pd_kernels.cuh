@@ -42,10 +42,22 @@ size_t kspace_smem_bytes(int W, int H);  // largest dynamic shared memory of the
 int gap_img_blocks(int W, int H, int T);
 cudaError_t configure_kernels();
 
-// one Cartesian iteration: dual, y-transform, rows, column adjoint, primal;
-// ev (optional) receives AVX_NSTAGE + 1 events around the stages
+// The dual update reads and writes nothing that the k-space stages touch (both
+// start from the extragradient), so a captured iteration runs it beside them.
+// fork: work on `side` from here on follows what `main` holds; join: `main`
+// goes on after what `side` holds.  Without a side stream both do nothing.
+struct SideStream {
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev = nullptr;
+  void fork(cudaStream_t main) const;
+  void join(cudaStream_t main) const;
+};
+
+// one Cartesian iteration: dual (on the side stream when there is one),
+// y-transform, rows, column adjoint, primal; ev (optional, without a side
+// stream) receives AVX_NSTAGE + 1 events around the stages
 void launch_iteration(int method, const PDArgs& a, const KArgs& k, float2* khz, cudaStream_t s,
-                      cudaEvent_t* ev = nullptr);
+                      const SideStream& side, cudaEvent_t* ev = nullptr);
 void launch_dual(int method, const PDArgs& a, cudaStream_t s);
 void launch_primal(int method, const PDArgs& a, cudaStream_t s);
 // the shape behind a tuning index: primal tile "TXxTYxYP", dual block "N threads"

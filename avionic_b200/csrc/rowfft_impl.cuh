@@ -50,7 +50,6 @@ __global__ void __launch_bounds__(320, 2) rowfft_kernel(KArgs a, int mode_rt, in
   using SP = RowSplit<N1, N2>;
   constexpr int W = SP::W, L = SP::L;
   const int mode = PD ? 0 : mode_rt;
-  if (a.st && a.st->stop && (PD || (mode != 3 && mode != 5))) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const CartGeomDev& g = a.g;
   const int C = g.C;
@@ -66,6 +65,9 @@ __global__ void __launch_bounds__(320, 2) rowfft_kernel(KArgs a, int mode_rt, in
     const int k1 = e / N2, j = e - k1 * N2;
     tw[e] = g.twx[k1 * j];
   }
+  pdl_wait();
+  pdl_trigger();
+  if (a.st && a.st->stop && (PD || (mode != 3 && mode != 5))) return;
   const int r = tid / L, l = tid - r * L;
   float2* row = buf + r * SP::ROW;
   const int sx = g.sx;
@@ -204,11 +206,11 @@ void rowfft_launch(const KArgs& k, int mode, cudaStream_t s) {
   const size_t sm = sizeof(float2) * (SP::W + (SP::W & 1) + (size_t)kc * (SP::ROW + (mode == 0 ? 2 * SP::W : 0)));
   const int nt = kc * SP::L;
   if (mode != 0)
-    rowfft_kernel<N1, N2, false, true><<<k.g.C * k.g.T, nt, sm, s>>>(k, mode, kc);
+    launch_dependent(rowfft_kernel<N1, N2, false, true>, k.g.C * k.g.T, nt, sm, s, k, mode, kc);
   else if (k.g.sx)
-    rowfft_kernel<N1, N2, true, true><<<k.g.C * k.g.T, nt, sm, s>>>(k, 0, kc);
+    launch_dependent(rowfft_kernel<N1, N2, true, true>, k.g.C * k.g.T, nt, sm, s, k, 0, kc);
   else
-    rowfft_kernel<N1, N2, true, false><<<k.g.C * k.g.T, nt, sm, s>>>(k, 0, kc);
+    launch_dependent(rowfft_kernel<N1, N2, true, false>, k.g.C * k.g.T, nt, sm, s, k, 0, kc);
 }
 
 template <int N1, int N2>

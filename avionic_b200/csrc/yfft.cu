@@ -67,13 +67,15 @@ AVX_D void load_maps(const float4* __restrict__ p, float2 (&m)[even(N1)]) {
 // 64 rows: 139 -> 27; 128 x 128, 20 frames, 8 coils, 16 rows: 20.7 -> 13.7.
 template <int N1>
 __global__ void __launch_bounds__(max_threads(N1)) yfft_kernel(KArgs a, int cpz) {
-  if (a.st && a.st->stop) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const CartGeomDev& g = a.g;
   const int W = g.W, H = g.H, C = g.C, n2 = H / N1;
   const int t = blockIdx.y;
   const int r0 = g.row_off[t], S = g.row_off[t + 1] - r0;
-  if (S == 0) return;
+  if (S == 0) {
+    pdl_wait();
+    return;
+  }
   constexpr int JP = (N1 + 1) * XT, E = even(N1);
   const int tid = threadIdx.x, nt = blockDim.x;  // nt = 32 tile_warps(n2) >= XT n2
   const int tx = tid & (XT - 1), j = tid / XT;
@@ -89,6 +91,9 @@ __global__ void __launch_bounds__(max_threads(N1)) yfft_kernel(KArgs a, int cpz)
     coef[p * pitch + (e - p * n2)] = a.yf_coef[(size_t)r0 * n2 + e];
   }
   for (int e = tid; e < S; e += nt) oc[e] = a.yf_order[r0 + e];
+  pdl_wait();
+  pdl_trigger();
+  if (a.st && a.st->stop) return;
   const int cb = blockIdx.z * cpz, ce = min(C, cb + cpz);
   const float4* __restrict__ maps =
       reinterpret_cast<const float4*>(a.b1t) +
@@ -161,7 +166,6 @@ __global__ void __launch_bounds__(max_threads(N1)) yfft_kernel(KArgs a, int cpz)
 // 2297 -> 433; 160 x 128 168 -> 41; 128 x 128 16.5 -> 15.4.
 template <int N1>
 __global__ void __launch_bounds__(max_threads(N1)) yfft_adj_kernel(KArgs a, float2* img, int groups) {
-  if (a.st && a.st->stop) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const CartGeomDev& g = a.g;
   const int W = g.W, H = g.H, C = g.C, n2 = H / N1;
@@ -185,6 +189,9 @@ __global__ void __launch_bounds__(max_threads(N1)) yfft_adj_kernel(KArgs a, floa
     const bool last = e + 1 == S || a.yf_order[r0 + e + 1].y != v.y;
     oc[e] = make_int2(v.x, last ? v.y * nt : -1);
   }
+  pdl_wait();
+  pdl_trigger();
+  if (a.st && a.st->stop) return;
   float2 acc[N1];
 #pragma unroll
   for (int i = 0; i < N1; ++i) acc[i] = cls[i * nt] = cls[(N1 + i) * nt] = czero();  // empty classes stay zero
@@ -309,20 +316,22 @@ __global__ void yfft_maps_kernel(const float2* __restrict__ b1, float2* __restri
     default: CALL(4); break;    \
   }
 
-// The longest register FFT that divides the height: each step down trades
+// The longest register FFT that divides the height and leaves n2 >= 4 (a
+// whole warp of 8 columns x n2 threads: 92 x 28, 19 coils, took 1.2 times as
+// long with n1 = 14, n2 = 2), else the longest at all: each step down trades
 // register butterflies for class sums.  At n1 = 4 the class sums are H / 4
 // long and the tensor-core partial DFT is faster where it applies (192 x 316,
 // 20 frames, 8 coils, 20 rows a frame: 93 us for both of its directions
 // against 117; n1 = 5 at 305 rows: 79 against 92), so 4 serves only the
 // frames with more rows than that form takes.
 int yfft_n1(int H, int max_rows) {
-  for (int n1 = 16; n1 >= (2 * max_rows > TC_MAX_NP ? 4 : 5); --n1) {
-    if (H % n1) continue;
-    const int n2 = H / n1;
-    if (32 * tile_warps(n2) > max_threads(n1)) continue;
-    if (fwd_smem(n1, n2, max_rows) > AVX_DYN_SMEM_MAX || adj_smem(n1, n2, max_rows, 1) > AVX_DYN_SMEM_MAX) continue;
-    return n1;
-  }
+  for (int least : {4, 1})
+    for (int n1 = 16; n1 >= (2 * max_rows > TC_MAX_NP ? 4 : 5); --n1) {
+      const int n2 = H / n1;
+      if (H % n1 || n2 < least || 32 * tile_warps(n2) > max_threads(n1)) continue;
+      if (fwd_smem(n1, n2, max_rows) > AVX_DYN_SMEM_MAX || adj_smem(n1, n2, max_rows, 1) > AVX_DYN_SMEM_MAX) continue;
+      return n1;
+    }
   return 0;
 }
 
@@ -364,7 +373,7 @@ void launch_yfft(const KArgs& k, cudaStream_t s) {
   const int cpz = 2 * ((k.g.C + 2 * z - 1) / (2 * z));
   dim3 gr(tiles, k.g.T, (k.g.C + cpz - 1) / cpz);
   const size_t sm = fwd_smem(k.yf_n1, n2, k.yf_rows);
-#define CALL_Y(N) yfft_kernel<N><<<gr, nt, sm, s>>>(k, cpz)
+#define CALL_Y(N) launch_dependent(yfft_kernel<N>, gr, nt, sm, s, k, cpz)
   YFFT_DISPATCH(k.yf_n1, CALL_Y)
 #undef CALL_Y
 }
@@ -379,7 +388,7 @@ void launch_yfft_adjoint(const KArgs& k, float2* img, cudaStream_t s) {
     grp *= 2;
   dim3 gr(tiles, k.g.T);
   const size_t sm = adj_smem(k.yf_n1, n2, k.yf_rows, grp);
-#define CALL_A(N) yfft_adj_kernel<N><<<gr, nt * grp, sm, s>>>(k, img, grp)
+#define CALL_A(N) launch_dependent(yfft_adj_kernel<N>, gr, nt * grp, sm, s, k, img, grp)
   YFFT_DISPATCH(k.yf_n1, CALL_A)
 #undef CALL_A
 }
