@@ -36,6 +36,7 @@
 #include "radial.cuh"
 #include "tc_dft.cuh"
 #include "utils_kernels.cuh"
+#include "radfft.cuh"
 #include "rowfft.cuh"
 #include "yfft.cuh"
 
@@ -268,6 +269,7 @@ avx_status configure_once() {
   AVX_CK(avx::configure_tc_kernels());
   AVX_CK(avx::configure_yfft_kernels());
   AVX_CK(avx::configure_rowfft_kernels());
+  AVX_CK(avx::configure_radfft_kernels());
   g_configured |= bit;
   return AVX_OK;
 }
@@ -527,6 +529,7 @@ static avx_status build_radial(avx_operator* op, const float* d_traj, const floa
   if (avx::radial_fft_smem_bytes(std::max(g.Gx, g.Gy)) > AVX_DYN_SMEM_MAX ||
       avx::radial_adj_smem_bytes(g.Gx, W) > AVX_DYN_SMEM_MAX)
     return fail(AVX_E_UNSUPPORTED, "oversampled grid too large for the grid FFT tile");
+  g.reg_fft = avx::radfft_applies(g) ? 1 : 0;
   std::vector<float2> twx(g.Gx), twy(g.Gy);
   for (int j = 0; j < g.Gx; ++j) twx[j] = make_float2((float)std::cos(2.0 * M_PI * j / g.Gx), (float)std::sin(2.0 * M_PI * j / g.Gx));
   for (int j = 0; j < g.Gy; ++j) twy[j] = make_float2((float)std::cos(2.0 * M_PI * j / g.Gy), (float)std::sin(2.0 * M_PI * j / g.Gy));
@@ -2780,7 +2783,7 @@ size_t request_workspace(const avx_request& r, long long R_known, int max_rows_k
   // solver: primal, extragradient and step scratch (3P), duals (D), z and d, reductions, history
   b += (3 * P + D) * N * c8 + 2 * kspace * c8;
   b += 8 * (size_t)std::max(AVX_RED_BLOCKS, avx::gap_img_blocks((int)W, (int)H, (int)T)) * 8;
-  b += 3 * (std::max(C * T, (kspace + 255) / 256) + 1) * 8;
+  b += 3 * (std::max(C * T * (r.op_kind == 1 ? (H * 4 + 31) / 32 + 1 : 1), (kspace + 255) / 256) + 1) * 8;
   b += 3 * ((size_t)r.params.maxIt + 3) * 8 + 4096;
   return b + b / 20 + ((size_t)4 << 20);  // pool granularity and slack
 }

@@ -1,0 +1,8 @@
+// Radial grid transforms (radfft_impl.cuh): grid sizes 130 to 176.
+#include "radfft_impl.cuh"
+
+namespace avx {
+
+RADFFT_DEFINE(b, RADFFT_SPLITS_B)
+
+}  // namespace avx

@@ -13,6 +13,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "fft.cuh"
+#include "radfft.cuh"
 #include "radial.cuh"
 
 namespace avx {
@@ -167,12 +168,16 @@ __global__ void __launch_bounds__(256) rad_fft_cols_kernel(RArgs a) {
   }
 }
 
-// window of one sample along one axis: start index (unwrapped) and weights
+// window of one sample along one axis (k cycles / pixel, grid size G): start
+// index (unwrapped) and weights.  The offsets kappa - g are formed by one
+// fused multiply-add from k: kappa = k G rounded first is off by up to half an
+// ulp of G / 2 (4e-6 grid cells at G = 192), which the window's slope turns
+// into an error of the same order in the weights.
 template <int NW>
-AVX_D int sample_window(float kappa, const RadialGeomDev& g, float (&w)[NW]) {
-  const int g0 = (int)floorf(kappa - 0.5f * g.J);
+AVX_D int sample_window(float k, float G, const RadialGeomDev& g, float (&w)[NW]) {
+  const int g0 = (int)floorf(k * G - 0.5f * g.J);
 #pragma unroll
-  for (int o = 0; o < NW; ++o) w[o] = kbw(kappa - (float)(g0 + o), g);
+  for (int o = 0; o < NW; ++o) w[o] = kbw(fmaf(k, G, -(float)(g0 + o)), g);
   return g0;
 }
 
@@ -182,8 +187,8 @@ __global__ void rad_window_kernel(RadialGeomDev g, int2* win0, float* winw) {
        i += (long long)gridDim.x * blockDim.x) {
     const int f = (int)(i / g.S), s = (int)(i % g.S);
     float wx[NW], wy[NW];
-    const int g0x = sample_window<NW>(g.traj[((long long)f * 2 + 0) * g.S + s] * (float)g.Gx, g, wx);
-    const int g0y = sample_window<NW>(g.traj[((long long)f * 2 + 1) * g.S + s] * (float)g.Gy, g, wy);
+    const int g0x = sample_window<NW>(g.traj[((long long)f * 2 + 0) * g.S + s], (float)g.Gx, g, wx);
+    const int g0y = sample_window<NW>(g.traj[((long long)f * 2 + 1) * g.S + s], (float)g.Gy, g, wy);
     win0[i] = make_int2(g0x, g0y);
 #pragma unroll
     for (int o = 0; o < NW; ++o) {
@@ -368,7 +373,9 @@ size_t radial_adj_smem_bytes(int G, int W) {
   return sizeof(float2) * (2 * (size_t)G * AVX_FFT_PITCH(RAD_ADJ_KC) + G + (size_t)RAD_ADJ_KC * W);
 }
 
-int radial_interp_blocks(const RadialGeomDev& g) { return (int)(((long long)g.T * g.C * g.S + 255) / 256); }
+int radial_interp_blocks(const RadialGeomDev& g) {
+  return g.reg_fft ? radfft_forward_blocks(g) : (int)(((long long)g.T * g.C * g.S + 255) / 256);
+}
 
 cudaError_t configure_radial_kernels() {
   cudaError_t e = cudaSuccess;
@@ -390,6 +397,10 @@ cudaError_t configure_radial_kernels() {
 
 // every FFT kernel runs 256 threads, as the compile-time plans assume
 void launch_rad_forward_grid(const RArgs& a, cudaStream_t s) {
+  if (a.g.reg_fft) {
+    launch_radfft_columns(a, s);
+    return;
+  }
   dim3 gr((a.g.Gy + RAD_FFT_KC - 1) / RAD_FFT_KC, a.g.C * a.g.T);
 #define CALL_F(ID) rad_rows_fwd_kernel<ID><<<gr, 256, radial_fft_smem_bytes(a.g.Gx), s>>>(a)
   AVX_FFT_PLAN_DISPATCH(fft_plan_id(a.g.Gx, a.g.nradx, a.g.radx), CALL_F)
@@ -401,6 +412,10 @@ void launch_rad_forward_grid(const RArgs& a, cudaStream_t s) {
 }
 
 void launch_rad_adjoint_image(const RArgs& a, float2* img, cudaStream_t s) {
+  if (a.g.reg_fft) {
+    launch_radfft_adjoint(a, img, s);
+    return;
+  }
   dim3 gc((a.g.Gx + RAD_FFT_KC - 1) / RAD_FFT_KC, a.g.C * a.g.T);
 #define CALL_C(ID) rad_fft_cols_kernel<ID, 1><<<gc, 256, radial_fft_smem_bytes(a.g.Gy), s>>>(a)
   AVX_FFT_PLAN_DISPATCH(fft_plan_id(a.g.Gy, a.g.nrady, a.g.rady), CALL_C)
@@ -423,6 +438,10 @@ void launch_rad_adjoint_image(const RArgs& a, float2* img, cudaStream_t s) {
   }
 
 void launch_rad_interp(const RArgs& a, int mode, cudaStream_t s) {
+  if (a.g.reg_fft) {
+    launch_radfft_interp(a, mode, s);
+    return;
+  }
   const int nb = radial_interp_blocks(a.g);
 #define CALL_I(N) rad_interp_kernel<N><<<nb, 256, 0, s>>>(a, mode)
   RAD_NW_DISPATCH(a.g.nw, CALL_I)

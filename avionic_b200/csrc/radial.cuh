@@ -30,6 +30,7 @@ struct RadialGeomDev {
   const float2* twgy;       // [Gy]
   int nradx, radx[12];      // FFT plan along x
   int nrady, rady[12];      // FFT plan along y
+  int reg_fft;              // the two-step register transforms of radfft.cuh apply
 };
 
 struct RArgs {
