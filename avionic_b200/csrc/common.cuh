@@ -73,6 +73,11 @@ struct DevState {
   double gap0;            // first normalised gap of the run (relative stop criterion)
 };
 
+namespace avx {
+// the library's stream-ordered memory pool on the current device (core.cu); null when it cannot be had
+cudaMemPool_t library_pool();
+}  // namespace avx
+
 // Programmatic dependent launch: a kernel launched with launch_dependent may
 // start while its predecessor still runs.  Until pdl_wait() it reads only what
 // no kernel writes (an operator's tables); pdl_wait() returns once the

@@ -71,7 +71,9 @@ thread_local cudaStream_t t_pool_stream = nullptr;
 // batch engine lives it keeps everything (pool_hold).  The attributes of the
 // application's default pool are never changed.
 constexpr unsigned long long kPoolKeep = 4ull << 30;
-static cudaMemPool_t library_pool() {
+}  // namespace
+namespace avx {
+cudaMemPool_t library_pool() {
   static std::mutex mu;
   static std::map<int, cudaMemPool_t> pools;
   int dev = 0;
@@ -92,6 +94,9 @@ static cudaMemPool_t library_pool() {
   pools[dev] = pool;
   return pool;
 }
+}  // namespace avx
+namespace {
+using avx::library_pool;
 
 template <class T>
 struct DevBuf {
@@ -500,17 +505,16 @@ static avx_status build_radial(avx_operator* op, const float* d_traj, const floa
   g.kb_norm = (float)(1.0 / (std::cyl_bessel_i(0.0, beta) - 1.0));
   g.norm = (float)(1.0 / std::sqrt((double)W * H));
   // deapodisation psi(p) = int w(t) cos(2 pi t p / G) dt
+  // (the kernel's values at the nodes once: evaluated per pixel and node they were 10 ms of an operator's creation)
   std::vector<double> gx, gw;
   gauss_legendre(64, gx, gw);
+  for (int i = 0; i < 64; ++i) gw[i] *= (J / 2.0) * kb_weight(gx[i] * J / 2.0, J, beta);
   auto deap = [&](int d, int G, std::vector<float>& inv) {
     inv.resize(d);
     for (int n = 0; n < d; ++n) {
       const double p = n - d / 2;
       double acc = 0.0;
-      for (int i = 0; i < 64; ++i) {
-        const double t = gx[i] * J / 2.0;
-        acc += gw[i] * (J / 2.0) * kb_weight(t, J, beta) * std::cos(2.0 * M_PI * t * p / G);
-      }
+      for (int i = 0; i < 64; ++i) acc += gw[i] * std::cos(2.0 * M_PI * (gx[i] * J / 2.0) * p / G);
       inv[n] = (float)(1.0 / acc);
     }
   };

@@ -542,7 +542,10 @@ __global__ void rad_iota_kernel(int* v, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] = i;
 }
 
-// stream-ordered scratch memory, returned on its stream when it goes out of scope
+// Stream-ordered scratch memory, returned on its stream when it goes out of
+// scope.  From the library's pool, which keeps freed memory: the device's
+// default pool unmaps it at the next synchronisation, so that building an
+// operator mapped its scratch anew each time (10 ms and more).
 struct AsyncScratch {
   void* p = nullptr;
   cudaStream_t s;
@@ -550,7 +553,10 @@ struct AsyncScratch {
   ~AsyncScratch() {
     if (p) cudaFreeAsync(p, s);
   }
-  cudaError_t alloc(size_t bytes) { return cudaMallocAsync(&p, bytes, s); }
+  cudaError_t alloc(size_t bytes) {
+    cudaMemPool_t pool = library_pool();
+    return pool ? cudaMallocFromPoolAsync(&p, bytes, pool, s) : cudaErrorMemoryAllocation;
+  }
   template <class T>
   T* as() const {
     return static_cast<T*>(p);
