@@ -58,6 +58,13 @@ void launch_absmax(const float2* v, int n, unsigned* out, cudaStream_t s);
 void launch_b1r_prep(const float2* u0, const unsigned* umax, const float2* crec, int coils, int HW, float tau,
                      float2* Lw, float2* Iu, cudaStream_t s);
 void launch_b1r_fused(const CoilPD& a, int coils, const B1Buffers& b, cudaStream_t s);
+// All iterations of a loop in one launch, each coil's image held by a cluster
+// of CTAs; false when the image does not fit one (the per-iteration kernels
+// then run the loop).  Start from zero fields (UTGV2: x1 from a.x1), results
+// in a.x1.
+bool launch_b1r_cluster(const CoilPD& a, int coils, unsigned iters, cudaStream_t s);
+bool launch_utgv_cluster(const CoilPD& a, unsigned iters, cudaStream_t s);
+cudaError_t configure_coil_kernels();
 void launch_b1r_normalize(const float2* x, float2* out, int HW, int coils, cudaStream_t s);
 void launch_phase_apply(const float2* absb1, const float2* x1, float2* out, int HW, cudaStream_t s);
 void launch_weight_update(float2* w, const float2* b, int HW, cudaStream_t s);

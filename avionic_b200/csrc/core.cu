@@ -275,6 +275,7 @@ avx_status configure_once() {
   AVX_CK(avx::configure_yfft_kernels());
   AVX_CK(avx::configure_rowfft_kernels());
   AVX_CK(avx::configure_radfft_kernels());
+  AVX_CK(avx::configure_coil_kernels());
   g_configured |= bit;
   return AVX_OK;
 }
@@ -1510,9 +1511,11 @@ avx_status coil_utgv2(int W, int H, const avx_coil_params& p, const float2* b10,
       ub[q].y2_out[k] = other(a.y2[k], 5 + k);
     }
   }
-  unsigned it = 0;
-  avx_status r = coil_iterate(l, p.uNrIt, s, [&] { avx::launch_utgv_fused(a, ub[it++ & 1u], s); });
-  if (r != AVX_OK) return r;
+  if (!avx::launch_utgv_cluster(a, p.uNrIt, s)) {
+    unsigned it = 0;
+    avx_status r = coil_iterate(l, p.uNrIt, s, [&] { avx::launch_utgv_fused(a, ub[it++ & 1u], s); });
+    if (r != AVX_OK) return r;
+  }
   AVX_CK(cudaMemcpyAsync(x1, l.xw.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, s));
   AVX_CK(cudaGetLastError());
   AVX_CK(cudaStreamSynchronize(s));
@@ -1556,7 +1559,7 @@ avx_status coil_b1_recon(int W, int H, int coils, unsigned max_it, float mu, con
   float2* ext2 = l.buf.p + 6 * CN;
   float2* y2[2] = {l.buf.p + 7 * CN, l.buf.p + 8 * CN};
   unsigned it = 0;
-  avx_status r = coil_iterate(l, max_it, s, [&] {
+  avx_status r = avx::launch_b1r_cluster(a, coils, max_it, s) ? AVX_OK : coil_iterate(l, max_it, s, [&] {
     const bool odd = (it++ & 1u) != 0;
     B1Buffers b;
     b.ext_in = odd ? ext2 : a.ext1;

@@ -137,3 +137,33 @@ def test_radial_operator_matches_oracle(W, H, C, osf, J):
     ig = op.forward(av.to_device(k), av.to_device(b1), out=torch.empty((T, H, W), dtype=torch.complex64,
                                                                      device="cuda")).cpu().numpy()
     assert _rel(ig, oop.forward(k.astype(complex), b1.astype(complex))) < REL_FFT
+
+
+# one CTA of the cluster holds 1 to 6 pixels a thread, uneven blocks of rows, an image of fewer rows than CTAs
+# (the per-iteration kernels), one too large for a cluster
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(40, 7), (33, 18), (64, 64), (128, 100), (160, 130), (200, 190), (330, 320)])
+@pytest.mark.parametrize("C", [1, 3])
+def test_coil_loops_match_oracle(W, H, C):
+    """UTGV2Recon, B1Recon and the H1 solve (fewer iterations than the defaults) against float64.  The loops are
+    contractions of fp32 values: 60 iterations add at most 60 roundings of 6e-8 coherently; 1e-5."""
+    import avionic_b200 as av
+    from oracle import coils as oc
+    rng = np.random.default_rng(W + H + C)
+    yy, xx = np.meshgrid(np.linspace(-1, 1, H), np.linspace(-1, 1, W), indexing="ij")
+    img = (np.exp(-3 * (yy ** 2 + xx ** 2)) + 0.2) * np.exp(1j * (xx + 0.5 * yy))
+    maps = np.stack([np.exp(-((yy - np.sin(c)) ** 2 + (xx - np.cos(c)) ** 2)) * np.exp(1j * c * xx) for c in range(C)])
+    crec = (maps * img + 0.01 * _cplx(rng, (C, H, W))).astype(np.complex64)
+    u = img.astype(np.complex64)
+    p = av.coil_default_params()
+    p.uNrIt = 60
+    q = oc.default_params()
+    q["uNrIt"] = 60
+    x1 = av.coil_utgv2(av.to_device(maps), av.to_device(crec), list(range(C)), av.to_device(u), params=p)
+    xo = oc.utgv2_recon(maps.astype(np.complex64).astype(complex), crec.astype(complex), u.astype(complex),
+                        list(range(C)), q)
+    assert _rel(x1.cpu().numpy(), xo) < 1e-5
+    b = av.coil_b1_recon(av.to_device(u), av.to_device(crec), C, 60, 2.0).cpu().numpy()
+    assert _rel(b, oc.b1_recon(u.astype(complex), crec.astype(complex), C, 60, 2.0, q)) < 1e-5
+    h = av.coil_b1_from_u_h1(av.to_device(u), av.to_device(crec)).cpu().numpy()
+    assert _rel(h, oc.b1_from_u_h1(u.astype(complex), crec.astype(complex), q)) < 1e-5
