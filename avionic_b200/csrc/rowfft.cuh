@@ -5,7 +5,8 @@
 
 namespace avx {
 
-// W = n1 n2 with 8 <= n2 <= n1 <= 16, or n1 = 20; false when W has no such split
+// W = n1 n2 with 8 <= n2 <= n1 <= 16, or n1 = 20, or one of the short splits
+// (rowfft_impl.cuh); false when W has no such split
 bool rowfft_split(int W, int* n1, int* n2);
 
 // the row kernel's work (launch_rows of pd_kernels.cuh) for a length with a

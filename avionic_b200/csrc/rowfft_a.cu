@@ -19,12 +19,16 @@ bool rowfft_split(int W, int* n1, int* n2) {
     *n2 = b;
     return true;
   }
-  return false;
+  return rowfft_short_split(W, n1, n2);
 }
 
 void launch_rowfft(const KArgs& k, int mode, cudaStream_t s) {
   int n1 = 0, n2 = 0;
   if (!rowfft_split(k.g.W, &n1, &n2)) return;
+  if (n2 < 8) {
+    rowfft_launch_short(n1, n2, k, mode, s);
+    return;
+  }
 #define CALL_W(N) \
   case N: rowfft_launch_##N(n2, k, mode, s); break;
   switch (n1) {
@@ -46,7 +50,7 @@ void launch_rowfft(const KArgs& k, int mode, cudaStream_t s) {
 cudaError_t configure_rowfft_kernels() {
   cudaError_t (*const all[])() = {rowfft_configure_8,  rowfft_configure_9,  rowfft_configure_10, rowfft_configure_11,
                                   rowfft_configure_12, rowfft_configure_13, rowfft_configure_14, rowfft_configure_15,
-                                  rowfft_configure_16, rowfft_configure_20};
+                                  rowfft_configure_16, rowfft_configure_20, rowfft_configure_short};
   for (auto f : all) {
     const cudaError_t e = f();
     if (e != cudaSuccess) return e;

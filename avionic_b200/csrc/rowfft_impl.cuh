@@ -224,6 +224,19 @@ cudaError_t rowfft_configure() {
   return e;
 }
 
+// Short rows (rowfft_e.cu): lengths 20 to 32 of 5 to 13 by 2 to 5 points, and
+// longer ones of 7 to 16 by 5 to 7.  Such a pass is all latency: two register
+// steps have one exchange where the Stockham plan has two to four, and the
+// kernel can be a dependent launch.  A whole TGV2 iteration, run-time plan and
+// here: 24 x 20, 6 frames, 4 coils 19.5 and 15.7 us; 50 x 64, 10 frames, 6
+// coils, 16 rows 33.3 and 19.2; 72 x 131, 12 frames, 8 coils 58.0 and 45.5;
+// 40 x 97, 10 frames, 8 coils 37.8 and 29.5.  Below 20 the plan's two steps
+// are as short, and other splits (an N2 under 5 at longer rows) leave most
+// lanes idle in one step.
+bool rowfft_short_split(int W, int* n1, int* n2);
+void rowfft_launch_short(int n1, int n2, const KArgs& k, int mode, cudaStream_t s);
+cudaError_t rowfft_configure_short();
+
 // one translation unit per first length, so that the instances build in parallel
 #define ROWFFT_DECLARE(N1)                                                       \
   void rowfft_launch_##N1(int n2, const KArgs& k, int mode, cudaStream_t s);     \

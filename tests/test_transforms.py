@@ -167,3 +167,11 @@ def test_coil_loops_match_oracle(W, H, C):
     assert _rel(b, oc.b1_recon(u.astype(complex), crec.astype(complex), C, 60, 2.0, q)) < 1e-5
     h = av.coil_b1_from_u_h1(av.to_device(u), av.to_device(crec)).cpu().numpy()
     assert _rel(h, oc.b1_from_u_h1(u.astype(complex), crec.astype(complex), q)) < 1e-5
+
+
+# short rows
+@pytest.mark.gpu
+@pytest.mark.parametrize("centered", [False, True])
+@pytest.mark.parametrize("W,rows", [(20, 5), (25, 17), (26, 16), (32, 3), (40, 8), (63, 13), (99, 9), (112, 20)])
+def test_short_row_transform_matches_oracle(W, rows, centered):
+    _check(W, 36, 3, 3, rows, centered, REL_FFT)
