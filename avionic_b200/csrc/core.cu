@@ -39,6 +39,7 @@
 #include "radfft.cuh"
 #include "rowfft.cuh"
 #include "yfft.cuh"
+#include "yfull.cuh"
 
 
 
@@ -273,6 +274,7 @@ avx_status configure_once() {
   AVX_CK(avx::configure_fft2d_kernels());
   AVX_CK(avx::configure_tc_kernels());
   AVX_CK(avx::configure_yfft_kernels());
+  AVX_CK(avx::configure_yfull_kernels());
   AVX_CK(avx::configure_rowfft_kernels());
   AVX_CK(avx::configure_radfft_kernels());
   AVX_CK(avx::configure_coil_kernels());
@@ -328,6 +330,10 @@ struct avx_operator {
   int yf_n1 = 0, max_rows = 0;
   DevBuf<int2> yf_order;
   DevBuf<float2> yf_coef;
+  // whole two-step y-transforms (yfull.cuh), when they are the faster ones; yf_n1 is then their first step
+  bool yfull = false;
+  DevBuf<int> yw_inv;
+  DevBuf<float2> yw_phase;
 
   CartGeomDev geom() const {
     CartGeomDev g;
@@ -402,8 +408,18 @@ static avx_status build_operator(avx_operator* op, const float* h_mask) {
   op->tc_np = max_rows > 0 && np <= TC_MAX_NP ? np : 0;
   op->dft_mode = op->tc_np ? AVX_DFT_SPLIT_BF16X3 : AVX_DFT_FP32;
   const int sy = op->centered ? H / 2 : 0;
-  op->yf_n1 = max_rows > 0 ? avx::yfft_n1(H, max_rows) : 0;
-  if (op->yf_n1) {
+  op->yf_n1 = max_rows > 0 ? avx::yfull_n1(W, H, T, max_rows) : 0;
+  op->yfull = op->yf_n1 != 0;
+  if (max_rows > 0 && !op->yfull) op->yf_n1 = avx::yfft_n1(H, max_rows);
+  if (op->yfull) {
+    std::vector<int> inv((size_t)T * H);
+    std::vector<float2> phase(H);
+    avx::yfull_build(H, T, sy, op->rows.data(), op->row_off.data(), inv.data(), phase.data());
+    AVX_CK(op->yw_inv.alloc(inv.size()));
+    AVX_CK(op->yw_phase.alloc(phase.size()));
+    AVX_CK(cudaMemcpy(op->yw_inv.p, inv.data(), inv.size() * sizeof(int), cudaMemcpyHostToDevice));
+    AVX_CK(cudaMemcpy(op->yw_phase.p, phase.data(), phase.size() * sizeof(float2), cudaMemcpyHostToDevice));
+  } else if (op->yf_n1) {
     const int n1 = op->yf_n1;
     std::vector<int2> order(op->R);
     std::vector<float2> coef((size_t)op->R * (H / n1));
@@ -943,6 +959,8 @@ static void set_dft(KArgs* k, const avx_operator* op) {
   k->yf_rows = op->max_rows;
   k->yf_order = op->yf_order.p;
   k->yf_coef = op->yf_coef.p;
+  k->yw_inv = op->yfull ? op->yw_inv.p : nullptr;
+  k->yw_phase = op->yw_phase.p;
   const bool on = uses_tc(op);
   k->tc_ytab = on ? op->tc_ytab.p : nullptr;
   k->tc_np = on ? op->tc_np : 0;
@@ -2777,6 +2795,8 @@ size_t request_workspace(const avx_request& r, long long R_known, int max_rows_k
     }
     if (const int n1 = max_rows > 0 ? avx::yfft_n1((int)H, (int)max_rows) : 0)
       b += R * (8 + H / n1 * 8) + avx::yfft_maps_count((int)W, (int)H, (int)C, n1) * c8;
+    if (const int n1 = max_rows > 0 ? avx::yfull_n1((int)W, (int)H, (int)T, (int)max_rows) : 0)
+      b += H * T * 4 + H * 8 + avx::yfft_maps_count((int)W, (int)H, (int)C, n1) * c8;
   } else {
     const size_t S = (size_t)r.n_fe * r.spokes_per_frame;
     const int isw = std::max(2, (int)r.sector_width);

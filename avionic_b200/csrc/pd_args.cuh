@@ -73,6 +73,9 @@ struct KArgs {
   int yf_n1, yf_rows;   // the FFT's length, the most sampled rows of a frame
   const int2* yf_order;
   const float2* yf_coef;
+  // whole two-step y-transforms (null: not used), tables of yfull.cuh
+  const int* yw_inv;
+  const float2* yw_phase;
   // row-FFT schedule of the row kernel (chosen by the autotuner): compact rows
   // per pass (8, 12 or 16; 0 = 16) and the radix plan (0: the compile-time
   // plan of the length when there is one, 1: the run-time plan)

@@ -20,6 +20,7 @@
 #include "tc_dft.cuh"
 #include "rowfft.cuh"
 #include "yfft.cuh"
+#include "yfull.cuh"
 
 namespace avx {
 
@@ -1337,6 +1338,10 @@ void launch_primal(int method, const PDArgs& a, cudaStream_t s) {
 }
 
 void launch_ydft(const KArgs& k, cudaStream_t s) {
+  if (k.yw_inv) {
+    launch_yfull(k, s);
+    return;
+  }
   if (k.yf_n1) {
     launch_yfft(k, s);
     return;
@@ -1379,6 +1384,10 @@ void launch_kspace(const KArgs& k, int mode, cudaStream_t s) {
 }
 
 void launch_adjoint(const KArgs& k, float2* img, cudaStream_t s) {
+  if (k.yw_inv) {
+    launch_yfull_adjoint(k, img, s);
+    return;
+  }
   if (k.yf_n1) {
     launch_yfft_adjoint(k, img, s);
     return;

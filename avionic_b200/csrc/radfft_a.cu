@@ -3,7 +3,7 @@
 
 namespace avx {
 
-RADFFT_DEFINE(a, RADFFT_SPLITS_A)
+RADFFT_DEFINE(a, FFT_SPLITS_A)
 
 static bool run(int G, int what, const RArgs* a, int mode, float2* img, cudaStream_t s) {
   return radfft_run_a(G, what, a, mode, img, s) || radfft_run_b(G, what, a, mode, img, s) ||

@@ -3,6 +3,6 @@
 
 namespace avx {
 
-RADFFT_DEFINE(b, RADFFT_SPLITS_B)
+RADFFT_DEFINE(b, FFT_SPLITS_B)
 
 }  // namespace avx

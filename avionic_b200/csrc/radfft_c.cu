@@ -3,6 +3,6 @@
 
 namespace avx {
 
-RADFFT_DEFINE(c, RADFFT_SPLITS_C)
+RADFFT_DEFINE(c, FFT_SPLITS_C)
 
 }  // namespace avx

@@ -3,6 +3,6 @@
 
 namespace avx {
 
-RADFFT_DEFINE(d, RADFFT_SPLITS_D)
+RADFFT_DEFINE(d, FFT_SPLITS_D)
 
 }  // namespace avx

@@ -17,6 +17,7 @@
 // 136 -> 63 with the spreading.
 #pragma once
 
+#include "fftsplits.cuh"
 #include "radfft.cuh"
 #include "regfft.cuh"
 
@@ -441,16 +442,6 @@ cudaError_t radfft_set() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(rad_rows_interp_kernel<N1, N2, 5>, dyn, AVX_DYN_SMEM_MAX);
   return e;
 }
-
-// splits of the grid sizes that image sizes of 64 to 160 give at oversampling
-// 1.5 and 2 (the smallest even sizes with factors up to 13), in four files
-#define RADFFT_SPLITS_A(X) X(12, 8) X(14, 7) X(10, 10) X(13, 8) X(12, 9) X(11, 10) X(14, 8) X(12, 10) X(14, 9) X(16, 8)
-#define RADFFT_SPLITS_B(X) \
-  X(13, 10) X(12, 11) X(14, 10) X(12, 12) X(15, 10) X(14, 11) X(13, 12) X(16, 10) X(18, 9) X(14, 12) X(16, 11)
-#define RADFFT_SPLITS_C(X) \
-  X(15, 12) X(14, 13) X(16, 12) X(14, 14) X(18, 11) X(20, 10) X(16, 13) X(15, 14) X(18, 12) X(20, 11) X(16, 14)
-#define RADFFT_SPLITS_D(X) \
-  X(18, 13) X(16, 15) X(18, 14) X(16, 16) X(20, 13) X(18, 15) X(20, 14) X(18, 16) X(20, 15) X(20, 16)
 
 #define RADFFT_DECLARE(F)                                                                              \
   bool radfft_run_##F(int G, int what, const RArgs* a, int mode, float2* img, cudaStream_t s);         \

@@ -169,6 +169,16 @@ def test_coil_loops_match_oracle(W, H, C):
     assert _rel(h, oc.b1_from_u_h1(u.astype(complex), crec.astype(complex), q)) < 1e-5
 
 
+# whole two-step column transforms (many sampled rows and enough columns for the grid), all rows, width tails, frames
+# without rows; at 2.5 n1 rows and just below, where the class sums take over
+@pytest.mark.gpu
+@pytest.mark.parametrize("centered", [False, True])
+@pytest.mark.parametrize("W,H,T,C,rows", [(250, 96, 12, 2, 96), (203, 98, 12, 1, 35), (203, 98, 12, 1, 34),
+                                          (160, 128, 20, 3, 64), (167, 162, 13, 2, 50), (250, 200, 9, 2, 60)])
+def test_column_transform_matches_oracle(W, H, T, C, rows, centered):
+    _check(W, H, C, T, rows, centered, REL_DENSE if W in (203, 167) else REL_FFT)
+
+
 # short rows
 @pytest.mark.gpu
 @pytest.mark.parametrize("centered", [False, True])
