@@ -4,9 +4,9 @@
 //                              column DFT -> interpolate
 // Adjoint  (samples -> image): spread (sector gather) -> column DFT (sign +1) ->
 //                              row DFT fused with crop+deapodise+coil-combine
-// The spreading step gathers: one CTA per (frame, sector) owns the sector's
-// grid cells and reads every sample of the 3x3 neighbouring sectors, so each
-// grid value is a fixed-order sum (no floating-point atomics, deterministic).
+// The spreading step gathers: a sector's grid cells have one owner, which
+// walks the list of the samples that reach the sector, so each grid value is a
+// fixed-order sum (no floating-point atomics, deterministic).
 #include <algorithm>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -15,6 +15,7 @@
 #include "fft.cuh"
 #include "radfft.cuh"
 #include "radial.cuh"
+#include "spread.cuh"
 
 namespace avx {
 
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(256) rad_interp_kernel(RArgs a, int mode) {
   }
 }
 
+// Sectors other than 8 x 8 cells, window widths outside 3 to 5 (else spread.cu):
 // one CTA per (sector, frame); thread = grid cell of the sector; CC coils
 // accumulated per pass over the sector's work list: the samples whose window
 // reaches the sector, in the order of the 3x3 neighbouring sectors and of the
@@ -661,6 +663,10 @@ void launch_rad_windows(const RadialGeomDev& g, int2* win0, float* winw, cudaStr
 }
 
 void launch_rad_spread(const RArgs& a, const float2* samples, cudaStream_t s) {
+  if (spread8_applies(a.g)) {
+    launch_spread8(a, samples, s);
+    return;
+  }
   const int grid = a.g.nsx * a.g.nsy * a.g.T;
   const int threads = a.g.sw * a.g.sw;
   // coils per pass: every pass re-reads the neighbouring sectors' samples

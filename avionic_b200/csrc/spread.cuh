@@ -1,0 +1,13 @@
+// Gridding of radial samples for sectors of 8 x 8 cells (spread.cu).
+#pragma once
+
+#include "radial.cuh"
+
+namespace avx {
+
+// the grid has sectors of 8 x 8 cells, windows of 3 to 5 points and sides of at least 32 cells
+bool spread8_applies(const RadialGeomDev& g);
+// launch_rad_spread of radial.cuh for such a grid
+void launch_spread8(const RArgs& a, const float2* samples, cudaStream_t s);
+
+}  // namespace avx

@@ -185,3 +185,29 @@ def test_column_transform_matches_oracle(W, H, T, C, rows, centered):
 @pytest.mark.parametrize("W,rows", [(20, 5), (25, 17), (26, 16), (32, 3), (40, 8), (63, 13), (99, 9), (112, 20)])
 def test_short_row_transform_matches_oracle(W, rows, centered):
     _check(W, 36, 3, 3, rows, centered, REL_FFT)
+
+
+# gridding by half sectors: several items a block (64 x 64, 90 frames), lists longer than a batch and empty ones, every
+# coil count's instance and a second pass over the coils, grids that the sectors do not divide, windows of 3 to 5 points;
+# the same tolerance as for the operator
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H,C,T,spokes,osf,J", [(64, 64, 1, 90, 1, 1.5, 3.0), (64, 60, 3, 1, 40, 2.0, 2.0),
+                                                  (21, 30, 5, 2, 9, 2.0, 3.0), (66, 64, 8, 2, 7, 1.5, 4.0),
+                                                  (45, 45, 12, 3, 1, 1.5, 3.0), (33, 50, 13, 2, 6, 2.0, 3.5),
+                                                  (64, 64, 17, 1, 30, 1.5, 3.0)])
+def test_gridding_matches_oracle(W, H, C, T, spokes, osf, J):
+    import torch
+
+    import avionic_b200 as av
+    from oracle.radial import RadialOperator as ORad
+    from oracle.radial import golden_angle_radial
+    rng = np.random.default_rng(W * 100 + C)
+    nfe = 2 * max(W, H) // 4 * 2
+    traj, dens = golden_angle_radial(nfe, spokes, T)
+    traj, dens = traj.astype(np.float32), dens.astype(np.float32)
+    b1, k = _cplx(rng, (C, H, W)), _cplx(rng, (T, C, spokes * nfe))
+    op = av.RadialOperator(W, H, C, T, av.to_device(traj), av.to_device(dens), spokes, J, 8.0, osf)
+    ig = op.forward(av.to_device(k), av.to_device(b1), out=torch.empty((T, H, W), dtype=torch.complex64,
+                                                                     device="cuda")).cpu().numpy()
+    oop = ORad(W, H, C, T, traj, dens, J, 8.0, osf)
+    assert _rel(ig, oop.forward(k.astype(complex), b1.astype(complex))) < REL_FFT
