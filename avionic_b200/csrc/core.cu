@@ -8,8 +8,8 @@
 // the verbose/debug/stop cadence.  All scalars that steer the loop (sigma,
 // tau, the gap, the stop flag) stay on the device, so iterations are
 // enqueued without host synchronisation; each of the four iteration shapes
-// (plain, +step, +gap, +step+gap) is captured once as a CUDA graph and
-// replayed.
+// (plain, +step, +gap, +step+gap) and a run of several plain iterations are
+// captured once as CUDA graphs and replayed.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -4,10 +4,14 @@
 // tgv2.cpp:234-335, ictgv2.cpp:334-490) with the Cartesian operator runs as
 // five kernels:
 //   dual_kernel    y <- prox(y + sigma * K_reg xbar)        (pointwise + stencils)
-//   ydft_kernel    y-transform of b1 xbar onto the sampled rows (all coils)
-//   rows_kernel    x-FFT of those rows, z <- prox(z + sigma (K xbar - d)),
-//                  Q' = row-IFFT(mask z); one CTA per (coil, frame)
-//   coladj_kernel  K^H z = sum_c conj(b1_c) column-IDFT(Q'_c)
+//   y-transform    of b1 xbar onto the sampled rows (all coils): yfull.cuh for
+//                  many rows, yfft.cuh else, and for heights without a factor
+//                  5 to 16 tc_dft.cuh or ydft_kernel here
+//   row pass       x-FFT of those rows, z <- prox(z + sigma (K xbar - d)),
+//                  Q' = row-IFFT(mask z): rowfft.cuh, or rows_kernel here for
+//                  widths without a two-step split; one CTA per (coil, frame)
+//   column adjoint K^H z = sum_c conj(b1_c) column-IDFT(Q'_c), by the
+//                  y-transform's form (coladj_kernel here)
 //   primal_kernel  divergence stencils, primal update and extragradient
 // The step-size rule (pd_recon.cpp:40-61) and the primal-dual gap
 // (tv.cpp:202-235, tgv2.cpp:130-176, ictgv2.cpp:163-249) are FP64 block
@@ -615,7 +619,7 @@ __global__ void __launch_bounds__(256, 4) rows_kernel(KArgs a, int mode) {
   constexpr int KCP = AVX_FFT_PITCH(KC);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const CartGeomDev& g = a.g;
-  const int W = PLAN > 1 ? PLAN : g.W, C = g.C;  // W compile-time with a fixed plan
+  const int W = g.W, C = g.C;
   const int c = blockIdx.x % C;
   const int t = blockIdx.x / C;
   const int r0 = g.row_off[t], r1 = g.row_off[t + 1];
@@ -1356,12 +1360,12 @@ void launch_ydft(const KArgs& k, cudaStream_t s) {
 
 template <int KC>
 static void launch_rows_kc(const KArgs& k, int mode, cudaStream_t s) {
-  // 256 threads, as the compile-time FFT plans assume
-  const int id = k.rows_rt ? fft_plan_id_runtime(k.g.nrad, k.g.rad) : fft_plan_id(k.g.W, k.g.nrad, k.g.rad);
+  const int id = fft_plan_id_runtime(k.g.nrad, k.g.rad);
   // launched in plain stream order: as a dependent launch its CTAs, resident early with up to 100 KB of shared
   // memory each, hold up what runs beside them (294 x 24, 4 coils: 50 us an iteration against 31)
 #define CALL_R(ID) rows_kernel<KC, ID><<<k.g.C * k.g.T, 256, rows_smem_bytes(k.g.W, KC), s>>>(k, mode)
-  AVX_FFT_PLAN_DISPATCH(id, CALL_R)
+  if (id == 1) CALL_R(1);
+  else CALL_R(0);
 #undef CALL_R
 }
 
@@ -1504,18 +1508,10 @@ cudaError_t configure_kernels() {
   // opt in to the full 227 KB of dynamic shared memory per CTA (sm_100)
   cudaError_t e = cudaFuncSetAttribute(ydft_kernel<KSPACE_KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);
   if (e != cudaSuccess) return e;
-  for (int id : {96, 128, 160, 192, 256, 320, 1, 0}) {
-#define SET_R(ID)                                                                                                  \
-  e = cudaFuncSetAttribute(rows_kernel<8, ID>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);       \
-  if (e == cudaSuccess)                                                                                            \
-    e = cudaFuncSetAttribute(rows_kernel<12, ID>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);    \
-  if (e == cudaSuccess)                                                                                            \
-    e = cudaFuncSetAttribute(rows_kernel<KSPACE_KC, ID>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX)
-    AVX_FFT_PLAN_DISPATCH(id, SET_R)
-#undef SET_R
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  for (auto f : {rows_kernel<8, 0>, rows_kernel<12, 0>, rows_kernel<KSPACE_KC, 0>, rows_kernel<8, 1>, rows_kernel<12, 1>,
+                 rows_kernel<KSPACE_KC, 1>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);
+  return e;
 }
 
 }  // namespace avx
