@@ -175,34 +175,6 @@ def load_peaks():
         return 6650.0, "fallback"
 
 
-def tensor_roofline(mask, W, H, T, C, ydft_ms, coladj_ms):
-    """Tensor-pipe roofline of the two split-BF16x3 kernels: the bf16 MMA FLOPs
-    they issue per launch (six piece products; tiles as tc_dft.cu launches
-    them: M = 128 (coil, column) pairs x N = 2 x rows per frame (padded to 16)
-    x K = 2H for the y-transform, M = 128 image rows x N = 16 coils x 8
-    columns x 2 x K = N' for the column adjoint) over the stage means, against
-    the sustained bf16 figure of MEASURED_PEAKS.json (kernels timed inside a
-    long reconstruction)."""
-    rows = max(int(np.count_nonzero(np.any(mask[t] != 0, axis=1))) for t in range(T))
-    npad = max(16, (2 * rows + 15) // 16 * 16)
-    ceil = lambda a, b: -(-a // b)  # noqa: E731
-    mma = lambda m, n, k: 2 * m * n * k  # noqa: E731
-    ydft = T * ceil(C * W, 128) * ceil(2 * H, 32) * 2 * 6 * mma(128, npad, 16)
-    coladj = T * ceil(H, 128) * ceil(W, 8) * sum(
-        (npad // 16) * 6 * mma(128, ceil(2 * 8 * min(16, C - c0), 16) * 16, 16) for c0 in range(0, C, 16))
-    try:
-        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-            peak, src = float(json.load(f)["bf16_tflops_sustained"]), "measured sustained"
-    except Exception:
-        peak, src = 1400.0, "fallback sustained"
-    out = {"peak_tflops": peak, "peak_source": src + " (MEASURED_PEAKS.json bf16_tflops_sustained)",
-           "n_per_mma_y_transform": npad}
-    for name, fl, ms in (("ydft_tc", ydft, ydft_ms), ("coladj_tc", coladj, coladj_ms)):
-        t = fl / (ms / 1000.0) / 1e12
-        out[name] = {"bf16_mma_gflop_per_launch": fl / 1e9, "achieved_tflops": t, "frac": t / peak}
-    return out
-
-
 def load_traffic():
     """DRAM bytes per launch by kernel from the committed ncu summary."""
     path = os.path.join(ROOT, "profiles", "kernel_traffic.txt")
@@ -655,7 +627,8 @@ def main():
     ap.add_argument("--cpu-iters", type=int, default=6)
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--dft", default="split", choices=["split", "fp32"],
-                    help="arithmetic of the y-transforms: split-BF16x3 tensor cores or fp32 CUDA cores")
+                    help="DFT mode of the Cartesian operator (heights without a factor 5 to 16: split-BF16x3 tensor "
+                         "cores or fp32 CUDA cores; other heights run fp32 register FFTs in either)")
     ap.add_argument("--parts", default="headline,tv128,radial,batched,serving",
                     help="comma list: headline (the 192x192x30 cine ICTGV2 line), tv128, radial, batched, serving "
                          "(added to the line at N=1; batched at every N)")
@@ -769,7 +742,8 @@ def main():
     assert torch.isfinite(torch.view_as_real(x)).all().item()
     err_oracle = vs_oracle("cine_192", x) if instance_seed(rank) == 1 else None
 
-    # the other arithmetic of the y-transforms, same problem and schedule (reported beside the headline)
+    # the operator's other DFT mode, same problem and schedule (reported beside the headline; at this height both
+    # modes run the fp32 register FFTs, so the images agree)
     other = None
     if args.dft == "split" and op.dft_mode == av.DFT_SPLIT_BF16X3:
         op.dft_mode = av.DFT_FP32
@@ -787,7 +761,7 @@ def main():
         g1.record()
         torch.cuda.synchronize()
         x_fp32 = x.clone()
-        other = {"dft": "fp32 CUDA cores", "value": job_rate(world, args.steps, max_over_ranks(dist, g0.elapsed_time(g1), "cuda")),
+        other = {"dft": "fp32", "value": job_rate(world, args.steps, max_over_ranks(dist, g0.elapsed_time(g1), "cuda")),
                  "unit": UNIT}
         op.dft_mode = av.DFT_SPLIT_BF16X3
         x.copy_(x0)
@@ -818,7 +792,7 @@ def main():
     achieved = ab[names[dom]] / (kmean[dom] / 1000.0) / 1e9
     traffic = load_traffic().get(names[dom])
     iter_ms = float(np.sum(kmean))
-    kern = {"dual": "dual_kernel", "ydft": "ydft_kernel", "rows": "rows_kernel", "coladj": "coladj_kernel",
+    kern = {"dual": "dual_kernel", "ydft": "yfft_kernel", "rows": "rowfft_kernel", "coladj": "yfft_adj_kernel",
             "primal": "primal_kernel"}
     roof = {"bound": "hbm", "kernel": kern[names[dom]], "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)"
@@ -830,8 +804,6 @@ def main():
             "iteration_algorithmic_bytes": ab["iteration"],
             "iteration_frac": ab["iteration"] / (iter_ms / 1000.0) / 1e9 / peak,
             "iteration_bytes_dense_layout": ab["iteration_dense_layout"]}
-    if args.dft == "split":
-        roof["tensor_kernels"] = tensor_roofline(prob["mask"], W, H, T, C, kmean[1], kmean[3])
 
     # end-to-end through the host-buffer entry point (pinned host buffers)
     pk = torch.from_numpy(prob["kdata"]).pin_memory()
@@ -885,8 +857,7 @@ def main():
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None,
-        "dtype": ("bf16x3-split y-DFTs on tensor cores (fp32 accumulate), f32 elsewhere" if args.dft == "split"
-                  else "f32 (complex64)"),
+        "dtype": "f32 (complex64)",
         "data": "synthetic",
         "config": CONFIG,
         "recons_per_s": value / ITERS,
@@ -895,7 +866,7 @@ def main():
                     "tuning": {"primal_tile": tuning[2], "dual_block_threads": tuning[3],
                                "dual_pixels_per_thread": 2 if tuning[1] >= 3 else 1,
                                "row_fft_rows_per_pass": row_schedule[0],
-                               "row_fft_plan": "run-time" if row_schedule[1] else "compile-time"},
+                               "row_fft_plan": "run-time" if row_schedule[1] else "two-step"},
                     "dft": args.dft, "other_dft_form": other,
                     "recon_latency_ms": {"p50": float(np.percentile(step_ms, 50)),
                                          "p99": float(np.percentile(step_ms, 99))}},

@@ -121,7 +121,9 @@ avx_status avx_cartesian_operator_create(unsigned width, unsigned height, unsign
  *                          accumulation; fp32-level accuracy)
  * Image heights with a factor of 5 to 16 (4 to 16 beyond 48 sampled rows per
  * frame) are transformed by fp32 register FFTs in either mode, which are both
- * faster and more accurate than the dense forms.  The split form needs at
+ * faster and more accurate than the dense forms (with many sampled rows as
+ * whole two-step FFTs, else with the sampled rows' sums over the FFT's
+ * classes).  The split form needs at
  * most 48 sampled rows per frame; otherwise AVX_E_UNSUPPORTED is returned and
  * the mode is unchanged.  New operators use the split form when it applies.
  * The radial operator ignores this. */
@@ -214,12 +216,11 @@ avx_status avx_solver_set_tuning(avx_solver* s, int autotune, int primal_tile, i
 avx_status avx_solver_get_tuning(const avx_solver* s, int* primal_tile, int* dual_block, const char** primal_name,
                                  int* dual_threads);
 /* FFT schedule of the Cartesian operator's row kernel: compact rows per pass
- * (8, 12 or 16; 16 by default) and the radix plan (0: the compile-time plan
- * of the row length when it has one, leading with radix-8 passes; 1: the
- * run-time plan).  With autotune set (avx_solver_set_tuning) the first run of
+ * (8, 12 or 16; 16 by default) and the radix plan (0: two register steps when
+ * the row length has such a split; 1, and other lengths: the run-time plan).  With autotune set (avx_solver_set_tuning) the first run of
  * a (device, method, W, H, T, C, sampled rows per frame) times the candidate
  * schedules on the solver's own fields and keeps the fastest, replacing what
- * is set here.  Rows per pass change the schedule only; the two radix plans
+ * is set here.  Rows per pass change the schedule only; the two plans
  * round differently (results agree to fp32 rounding). */
 avx_status avx_solver_set_kspace_schedule(avx_solver* s, int rows_per_pass, int runtime_plan);
 avx_status avx_solver_get_kspace_schedule(const avx_solver* s, int* rows_per_pass, int* runtime_plan);
