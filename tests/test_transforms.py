@@ -187,14 +187,15 @@ def test_short_row_transform_matches_oracle(W, rows, centered):
     _check(W, 36, 3, 3, rows, centered, REL_FFT)
 
 
-# gridding by half sectors: several items a block (64 x 64, 90 frames), lists longer than a batch and empty ones, every
+# gridding by half sectors: several items a warp (64 x 64, 67 and 90 frames) or shared long lists, lists longer than a batch and empty ones, every
 # coil count's instance and a second pass over the coils, grids that the sectors do not divide, windows of 3 to 5 points;
 # the same tolerance as for the operator
 @pytest.mark.gpu
 @pytest.mark.parametrize("W,H,C,T,spokes,osf,J", [(64, 64, 1, 90, 1, 1.5, 3.0), (64, 60, 3, 1, 40, 2.0, 2.0),
                                                   (21, 30, 5, 2, 9, 2.0, 3.0), (66, 64, 8, 2, 7, 1.5, 4.0),
                                                   (45, 45, 12, 3, 1, 1.5, 3.0), (33, 50, 13, 2, 6, 2.0, 3.5),
-                                                  (64, 64, 17, 1, 30, 1.5, 3.0)])
+                                                  (64, 64, 17, 1, 30, 1.5, 3.0), (64, 64, 5, 67, 1, 1.5, 3.0),
+                                                  (64, 64, 17, 67, 1, 1.5, 3.0)])
 def test_gridding_matches_oracle(W, H, C, T, spokes, osf, J):
     import torch
 
