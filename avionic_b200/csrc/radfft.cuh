@@ -1,4 +1,4 @@
-// Grid transforms of the radial operator with two-step register FFTs (radfft.cu).
+// Grid transforms of the radial operator with two-step register FFTs (radfft_impl.cuh).
 #pragma once
 
 #include "radial.cuh"

@@ -14,7 +14,7 @@
 // of 256 samples, grid 192 x 192: forward transform and interpolation 252 ->
 // 148 us, adjoint transform 176 -> 98; 104 x 90, 23 frames, 5 coils, 13 spokes
 // of 208, grid 208 x 180 (a run-time plan with radix 13 before): 107 -> 47 and
-// 136 -> 63 with the spreading.
+// 136 -> 55 with the spreading (of spread.cu).
 #pragma once
 
 #include "fftsplits.cuh"

@@ -64,7 +64,7 @@ AVX_D void load_maps(const float4* __restrict__ p, float2 (&m)[even(N1)]) {
 // instructions to 14.7 M (40.6 -> 32.4 us).  Cine: 52.7 us with the
 // tensor-core partial DFT, 32.4 here; 320 x 320, 48 frames, 32 coils, 53 rows:
 // 2332 us with the dense fp32 sums, 319 here; 160 x 128, 24 frames, 12 coils,
-// 64 rows: 139 -> 27; 128 x 128, 20 frames, 8 coils, 16 rows: 20.7 -> 13.7.
+// 64 rows: 139 -> 27 (23 by yfull_impl.cuh, which takes it); 128 x 128, 20 frames, 8 coils, 16 rows: 20.7 -> 13.7.
 template <int N1>
 __global__ void __launch_bounds__(max_threads(N1)) yfft_kernel(KArgs a, int cpz) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
