@@ -110,7 +110,8 @@ inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t
 #define AVX_RED_SLOTS 12
 #define AVX_RED_BLOCKS 592  // 4 x 148 SMs
 
-// Block-wide sum of NS doubles; results valid in thread 0.
+// Block-wide sum of NS doubles; results valid in thread 0.  The block has
+// whole warps: a shuffle from a lane that does not exist is undefined.
 template <int NS>
 AVX_D void block_sum(double (&v)[NS], double* smem /* >= 32*NS */) {
   const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);

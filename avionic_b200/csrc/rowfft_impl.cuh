@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(320, 2) rowfft_kernel(KArgs a, int mode_rt, in
   float2* buf = tw + W + (W & 1);                    // [kc][ROW]
   float2* zs = buf + kc * SP::ROW;                   // PD: [kc][W] of z, then of d
   float2* ds = zs + kc * W;
-  const int tid = threadIdx.x;  // kc L threads
+  const int tid = threadIdx.x;  // kc L threads, and idle ones up to a whole warp
   for (int e = tid; e < W; e += blockDim.x) {
     const int k1 = e / N2, j = e - k1 * N2;
     tw[e] = g.twx[k1 * j];
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(320, 2) rowfft_kernel(KArgs a, int mode_rt, in
   double acc[3] = {0.0, 0.0, 0.0};
   for (int k0 = 0; k0 < S; k0 += kc) {
     const int kk = k0 + r;
-    const bool live = kk < S;
+    const bool live = r < kc && kk < S;
     const long long base = zb + (long long)kk * W;
     const bool first = live && l < N2, second = live && l < N1;
     __syncthreads();  // the twiddles are staged; the previous pass has read its rows
@@ -204,7 +204,7 @@ void rowfft_launch(const KArgs& k, int mode, cudaStream_t s) {
   using SP = RowSplit<N1, N2>;
   const int kc = k.rows_kc ? k.rows_kc : 16;  // rows per pass: 8, 12 or 16
   const size_t sm = sizeof(float2) * (SP::W + (SP::W & 1) + (size_t)kc * (SP::ROW + (mode == 0 ? 2 * SP::W : 0)));
-  const int nt = kc * SP::L;
+  const int nt = (kc * SP::L + 31) / 32 * 32;  // block_sum's shuffles need whole warps
   if (mode != 0)
     launch_dependent(rowfft_kernel<N1, N2, false, true>, k.g.C * k.g.T, nt, sm, s, k, mode, kc);
   else if (k.g.sx)

@@ -212,3 +212,41 @@ def test_gridding_matches_oracle(W, H, C, T, spokes, osf, J):
                                                                      device="cuda")).cpu().numpy()
     oop = ORad(W, H, C, T, traj, dens, J, 8.0, osf)
     assert _rel(ig, oop.forward(k.astype(complex), b1.astype(complex))) < REL_FFT
+
+
+# row lengths whose threads do not fill whole warps (first lengths 5, 11, 13 and 15), at each number of rows a pass
+@pytest.mark.gpu
+@pytest.mark.parametrize("kc", [8, 12, 16])
+@pytest.mark.parametrize("W", [20, 99, 104, 150])
+def test_row_sums_match_oracle(W, kc):
+    """The sums of the step rule and of the gap, which the row kernel adds up over a block: 21 ICTGV2 iterations
+    (its step rule lowers sigma and tau early; the stop test evaluates the gap at the 21st).  A sum of squares of
+    values good to 2e-6 is good to 4e-6, and sigma and tau are roots of ratios of such sums: 1e-5; the gap adds
+    eight sums without cancellation this early: 2e-5."""
+    import torch
+
+    import avionic_b200 as av
+    from avionic_b200 import synth
+    from oracle import solvers as so
+    prob = synth.small(W, H=28, W=W, T=3, C=3)
+    T, C, H, _ = prob["kdata"].shape
+    op = av.CartesianOperator(W, H, C, T, mask=av.to_device(prob["mask"]), centered=False)
+    s = av.Solver("ICTGV2", op)
+    p = s.params
+    p.maxIt, p.stopPDGap = 21, 1e-30
+    s.params = p
+    s.set_tuning(False, 0, 0)
+    s.set_kspace_schedule(kc, False)
+    x = torch.zeros((T, H, W), dtype=torch.complex64, device="cuda")
+    s.run(av.to_device(prob["kdata"]), x, av.to_device(prob["b1"]))
+    oop = OCart(W, H, C, T, mask=prob["mask"], centered=False)
+    q = so.init_params("ICTGV2")
+    q.lam = oop.adapt_lambda(*q.adapt_kd)
+    q.maxIt, q.stopPDGap = 21, 1e-30
+    tr = {}
+    so.run("ICTGV2", prob["kdata"].astype(complex), np.zeros((T, H, W), complex), prob["b1"].astype(complex), oop, q, tr)
+    st = s.stats()
+    assert tr["steps"][-1][0] < 0.99 * q.sigma  # the rule has acted
+    assert abs(st.sigma - tr["steps"][-1][0]) < 1e-5 * st.sigma
+    assert abs(st.tau - tr["steps"][-1][1]) < 1e-5 * st.tau
+    assert abs(st.last_gap - tr["PDGap"][-1]) < 2e-5 * tr["PDGap"][-1]
