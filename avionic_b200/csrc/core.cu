@@ -309,9 +309,14 @@ struct avx_operator {
   int S = 0, spf = 0;
   RadialGeomDev rg{};
   DevBuf<float> r_traj, r_sqrtw, r_ipx, r_ipy;
-  DevBuf<int> r_order, r_secstart, r_spread_list, r_spread_off, r_spread_blocks;
-  DevBuf<int2> r_win0;
-  DevBuf<float> r_winw;
+  DevBuf<int> r_order, r_secstart;
+  // the samples' windows and the spreading's work lists; r_base: those of the
+  // baseline iterations (baseline_iter)
+  struct RadTables {
+    DevBuf<int2> win0;
+    DevBuf<float> winw;
+    DevBuf<int> list, off, blocks;
+  } r_tab, r_base;
   DevBuf<float2> r_twgx, r_twgy, r_grid;
   DevBuf<float2> r_khz;  // K^H z image (T x H x W), both operator kinds
   bool has_mask = false, binary = true;
@@ -334,6 +339,9 @@ struct avx_operator {
   bool yfull = false;
   DevBuf<int> yw_inv;
   DevBuf<float2> yw_phase;
+  // the tables of the baseline iterations (baseline_iter), built by the first run that has some (ensure_baseline)
+  std::mutex base_mu;
+  bool base_ready = false;
 
   CartGeomDev geom() const {
     CartGeomDev g;
@@ -352,6 +360,20 @@ struct avx_operator {
     return g;
   }
 };
+
+// coefficient tables of the tensor-core transforms (at most 48 rows per frame)
+static avx_status build_tc_tables(avx_operator* op) {
+  const int W = op->W, H = op->H, T = op->T, np = op->tc_np, sx = op->centered ? W / 2 : 0, sy = op->centered ? H / 2 : 0;
+  std::vector<unsigned short> tab(avx::tc_ytab_bytes(H, T, np) / 2);
+  avx::tc_build_ytab(W, H, T, sx, sy, op->rows.data(), op->row_off.data(), np, tab.data());
+  AVX_CK(op->tc_ytab.alloc(tab.size() * 2 / sizeof(uint4)));
+  AVX_CK(cudaMemcpy(op->tc_ytab.p, tab.data(), tab.size() * 2, cudaMemcpyHostToDevice));
+  std::vector<unsigned short> ctab(avx::tc_ctab_bytes(H, T, np) / 2);
+  avx::tc_build_ctab(H, T, sy, op->rows.data(), op->row_off.data(), np, ctab.data());
+  AVX_CK(op->tc_ctab.alloc(ctab.size() * 2 / sizeof(uint4)));
+  AVX_CK(cudaMemcpy(op->tc_ctab.p, ctab.data(), ctab.size() * 2, cudaMemcpyHostToDevice));
+  return AVX_OK;
+}
 
 static avx_status build_operator(avx_operator* op, const float* h_mask) {
   const int W = op->W, H = op->H, T = op->T;
@@ -429,15 +451,7 @@ static avx_status build_operator(avx_operator* op, const float* h_mask) {
     AVX_CK(cudaMemcpy(op->yf_order.p, order.data(), order.size() * sizeof(int2), cudaMemcpyHostToDevice));
     AVX_CK(cudaMemcpy(op->yf_coef.p, coef.data(), coef.size() * sizeof(float2), cudaMemcpyHostToDevice));
   } else if (op->tc_np) {
-    // coefficient tables of the tensor-core transforms (at most 48 rows per frame)
-    std::vector<unsigned short> tab(avx::tc_ytab_bytes(H, T, np) / 2);
-    avx::tc_build_ytab(W, H, T, op->centered ? W / 2 : 0, sy, op->rows.data(), op->row_off.data(), np, tab.data());
-    AVX_CK(op->tc_ytab.alloc(tab.size() * 2 / sizeof(uint4)));
-    AVX_CK(cudaMemcpy(op->tc_ytab.p, tab.data(), tab.size() * 2, cudaMemcpyHostToDevice));
-    std::vector<unsigned short> ctab(avx::tc_ctab_bytes(H, T, np) / 2);
-    avx::tc_build_ctab(H, T, sy, op->rows.data(), op->row_off.data(), np, ctab.data());
-    AVX_CK(op->tc_ctab.alloc(ctab.size() * 2 / sizeof(uint4)));
-    AVX_CK(cudaMemcpy(op->tc_ctab.p, ctab.data(), ctab.size() * 2, cudaMemcpyHostToDevice));
+    return build_tc_tables(op);
   }
   return AVX_OK;
 }
@@ -483,6 +497,35 @@ static int radial_grid_size(int d, double osf) {
   int n = 2 * (int)std::ceil(osf * d / 2.0);
   while (!smooth13(n)) n += 2;
   return n;
+}
+
+// The samples' windows and the spreading's work lists of g's samples, into
+// tables t (and into g).  Per (frame, sector), the samples whose window
+// reaches the sector's cells, in the order the sector sums them: the 3x3
+// neighbouring sectors in (dy, dx) order, each in sorted order (fewer than
+// three sectors along an axis wrap onto themselves and are taken once).
+// The CTAs are numbered heaviest list first, so that the central sectors,
+// which every spoke crosses, start in the first wave.
+static avx_status build_rad_tables(const avx_operator* op, bool rounded, avx_operator::RadTables& t, RadialGeomDev& g) {
+  const size_t n = (size_t)g.T * g.S, nsec = (size_t)g.T * g.nsx * g.nsy;
+  // the samples' window starts and weights depend on the trajectory alone
+  AVX_CK(t.win0.alloc(n));
+  AVX_CK(t.winw.alloc(n * 2 * g.nw));
+  avx::launch_rad_windows(g, rounded, t.win0.p, t.winw.p, 0);
+  AVX_CK(cudaGetLastError());
+  AVX_CK(cudaStreamSynchronize(0));
+  g.win0 = t.win0.p;
+  g.winw = t.winw.p;
+  AVX_CK(t.off.alloc(nsec + 1));
+  long long total = 0;
+  AVX_CK(avx::rad_count_lists(g, op->r_order.p, op->r_secstart.p, t.win0.p, t.off.p, &total, 0));
+  AVX_CK(t.list.alloc(std::max<size_t>((size_t)total, 1)));
+  AVX_CK(t.blocks.alloc(nsec));
+  AVX_CK(avx::rad_fill_lists(g, op->r_order.p, op->r_secstart.p, t.win0.p, t.off.p, t.list.p, t.blocks.p, 0));
+  g.spread_list = t.list.p;
+  g.spread_off = t.off.p;
+  g.spread_blocks = t.blocks.p;
+  return AVX_OK;
 }
 
 // The gridding operator's tables.  d_traj [T][2][S] and d_dens [T][S] are
@@ -579,39 +622,41 @@ static avx_status build_radial(avx_operator* op, const float* d_traj, const floa
   g.sec_start = op->r_secstart.p;
   g.twgx = op->r_twgx.p;
   g.twgy = op->r_twgy.p;
-  // the samples' window starts and weights depend on the trajectory alone
-  AVX_CK(op->r_win0.alloc((size_t)T * S));
-  AVX_CK(op->r_winw.alloc((size_t)T * S * 2 * g.nw));
-  avx::launch_rad_windows(g, op->r_win0.p, op->r_winw.p, 0);
-  AVX_CK(cudaGetLastError());
-  AVX_CK(cudaStreamSynchronize(0));
-  g.win0 = op->r_win0.p;
-  g.winw = op->r_winw.p;
-  // The spreading's work list.  Per (frame, sector), the samples whose window
-  // reaches the sector's cells, in the order the sector sums them: the 3x3
-  // neighbouring sectors in (dy, dx) order, each in sorted order (fewer than
-  // three sectors along an axis wrap onto themselves and are taken once).
-  // The CTAs are numbered heaviest list first, so that the central sectors,
-  // which every spoke crosses, start in the first wave.
-  {
-    AVX_CK(op->r_spread_off.alloc((size_t)T * nsec + 1));
-    long long total = 0;
-    AVX_CK(avx::rad_count_lists(g, op->r_order.p, op->r_secstart.p, op->r_win0.p, op->r_spread_off.p, &total, 0));
-    AVX_CK(op->r_spread_list.alloc(std::max<size_t>((size_t)total, 1)));
-    AVX_CK(op->r_spread_blocks.alloc((size_t)T * nsec));
-    AVX_CK(avx::rad_fill_lists(g, op->r_order.p, op->r_secstart.p, op->r_win0.p, op->r_spread_off.p,
-                               op->r_spread_list.p, op->r_spread_blocks.p, 0));
-    g.spread_list = op->r_spread_list.p;
-    g.spread_off = op->r_spread_off.p;
-    g.spread_blocks = op->r_spread_blocks.p;
-  }
-  return AVX_OK;
+  return build_rad_tables(op, false, op->r_tab, g);
 }
 
-static RArgs make_rargs(avx_operator* op, const float2* b1, const float2* in, const float2* in2) {
+// an operator's geometry for the baseline iterations (baseline_iter)
+static RadialGeomDev baseline_geom(const avx_operator* op) {
+  RadialGeomDev g = op->rg;
+  g.reg_fft = 0;
+  g.per_sector = 1;
+  g.win0 = op->r_base.win0.p;
+  g.winw = op->r_base.winw.p;
+  g.spread_list = op->r_base.list.p;
+  g.spread_off = op->r_base.off.p;
+  g.spread_blocks = op->r_base.blocks.p;
+  return g;
+}
+
+// builds what the baseline iterations (baseline_iter) read and no others do
+static avx_status ensure_baseline(avx_operator* op) {
+  std::lock_guard<std::mutex> lk(op->base_mu);
+  if (op->base_ready) return AVX_OK;
+  avx_status r = AVX_OK;
+  if (op->kind == 1) {
+    RadialGeomDev g = op->rg;
+    r = build_rad_tables(op, true, op->r_base, g);
+  } else if (op->tc_np && op->yf_n1) {  // else there already
+    r = build_tc_tables(op);
+  }
+  op->base_ready = r == AVX_OK;
+  return r;
+}
+
+static RArgs make_rargs(avx_operator* op, const float2* b1, const float2* in, const float2* in2, bool base = false) {
   RArgs r;
   memset(&r, 0, sizeof(r));
-  r.g = op->rg;
+  r.g = base ? baseline_geom(op) : op->rg;
   r.b1 = b1;
   r.in = in;
   r.in2 = in2;
@@ -682,15 +727,16 @@ struct avx_solver {
   bool own_stream = false;  // stream created by solver_alloc (else lent by the batch engine)
   // device state
   DevBuf<float2> prim, ext, dual, escr, z, d;
-  DevBuf<float2> b1t;  // coil maps in the y-transforms' order (order_maps)
+  DevBuf<float2> b1t, b1t_base;  // coil maps in the y-transforms' order (order_maps), baseline iterations' apart
   DevBuf<DevState> st;
   DevBuf<double> pimg, pk, hist;
   int cap = 0;
   double d_off_energy = 0.0;
   avx_run_stats stats{};
   DevState last{};
-  // graphs of the four iteration shapes, and of kChunk plain iterations in a row
-  cudaGraphExec_t gexec[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  // graphs of the four iteration shapes and of kChunk plain iterations in a
+  // row, with the operator's transforms and with the baseline ones
+  cudaGraphExec_t gexec[2][5] = {};
   // streams the graphs are captured on, whose priorities their kernels take:
   // the k-space stages and the primal update before the dual update beside them
   cudaStream_t capture = nullptr;
@@ -711,11 +757,12 @@ struct avx_solver {
     if (capture) cudaStreamDestroy(capture);
   }
   void drop_graphs() {
-    for (auto& g : gexec)
-      if (g) {
-        cudaGraphExecDestroy(g);
-        g = nullptr;
-      }
+    for (auto& form : gexec)
+      for (auto& g : form)
+        if (g) {
+          cudaGraphExecDestroy(g);
+          g = nullptr;
+        }
   }
   long long N() const { return (long long)W * H * T; }
   float2* primc(int c) { return prim.p + (size_t)c * N(); }
@@ -723,6 +770,34 @@ struct avx_solver {
   float2* dualc(int c) { return dual.p + (size_t)c * N(); }
   float2* escrc(int c) { return escr.p + (size_t)c * N(); }
 };
+
+// Iterations whose transforms stay the baseline ones: the dense or
+// split-BF16x3 y-transforms and Stockham rows, on radial grids the Stockham
+// passes, windows from rounded coordinates and gridding by whole sectors.
+// They are slower, but the image depends on which rounding is used:
+//  - TGV2 starts at step sizes above what the norm of its operator allows, and
+//    its step rule corrects them at k = 50 (before, the modes that grow are
+//    too small to be seen).  Until then the loop amplifies rounding: two
+//    operators, both within 1e-6 of float64, give images 6e-5 apart after 40
+//    iterations and 2e-4 after 50 (96 x 96, 32 frames, 19 coils), which then
+//    agree again (2e-6 after 500).
+//  - ICTV's step rule leaves out the regulariser (ictv.cpp) and never corrects
+//    them: 1e-4 after 10 iterations, 4e-3 after 200 (160 x 160, 20 frames).
+//  - The reported gap is the difference of sums that come to agree: the split
+//    form's truncation, 2e-6 in a TV image, is 4e-5 in its gap (96 x 96, 450
+//    iterations).
+// A result there is as reproducible as its rounding, so that is not changed
+// for speed.  TV, TVtemp and ICTGV2 (whose rule acts within ten iterations)
+// agree to 1e-5 at most between the two.
+static bool baseline_iter(const avx_solver* s, unsigned k) {
+  return (s->debug && s->debugstep > 0) || s->method == AVX_METHOD_ICTV || (s->method == AVX_METHOD_TGV2 && k <= 50);
+}
+
+// partial sums of one k-space pass
+static int kspace_blocks(const avx_operator* op, bool base) {
+  if (op->kind == 0) return op->C * op->T;
+  return avx::radial_interp_blocks(base ? baseline_geom(op) : op->rg);
+}
 
 static avx_status solver_alloc(avx_solver* s) {
   const int P = method_P(s->method), D = method_D(s->method);
@@ -736,7 +811,7 @@ static avx_status solver_alloc(avx_solver* s) {
   AVX_CK(s->d.alloc(K));
   AVX_CK(s->st.alloc(1));
   AVX_CK(s->pimg.alloc((size_t)8 * std::max(AVX_RED_BLOCKS, avx::gap_img_blocks(s->W, s->H, s->T))));
-  const int nk = s->op->kind == 1 ? avx::radial_interp_blocks(s->op->rg) : s->C * s->T;
+  const int nk = std::max(kspace_blocks(s->op, false), kspace_blocks(s->op, true));
   AVX_CK(s->pk.alloc((size_t)3 * std::max(nk, 1)));
   s->cap = (int)s->p.maxIt + 2;
   AVX_CK(s->hist.alloc((size_t)3 * (s->cap + 1)));
@@ -834,7 +909,7 @@ static avx_status time_launches(avx_solver* s, void (*launch)(int, const PDArgs&
   return AVX_OK;
 }
 
-static KArgs make_kargs(avx_solver* s, const float2* b1, const float2* in, const float2* in2);
+static KArgs make_kargs(avx_solver* s, const float2* b1, const float2* in, bool base);
 
 // Row-FFT schedules the tuner tries: rows per pass (8, 12, 16) with the
 // compile-time radix plan of the length, and 16 rows per pass with the
@@ -842,7 +917,7 @@ static KArgs make_kargs(avx_solver* s, const float2* b1, const float2* in, const
 // change the schedule only (every sequence goes through the same passes); the
 // two radix plans round differently.
 static avx_status tune_rows(avx_solver* s, const float2* b1) {
-  KArgs k = make_kargs(s, b1, s->extc(0), nullptr);
+  KArgs k = make_kargs(s, b1, s->extc(0), baseline_iter(s, s->p.maxIt));
   const CartGeomDev& g = k.g;
   const bool has_fixed = fft_plan_id(g.W, g.nrad, g.rad) != fft_plan_id_runtime(g.nrad, g.rad);
   const int cand[4][2] = {{KSPACE_KC, 0}, {12, 0}, {8, 0}, {KSPACE_KC, 1}};
@@ -950,31 +1025,31 @@ static avx_status autotune(avx_solver* s, const float2* b1) {
 }
 
 // the split form runs on the tensor cores
-static bool uses_tc(const avx_operator* op) {
-  return op->kind == 0 && op->dft_mode == AVX_DFT_SPLIT_BF16X3 && op->tc_np > 0 && !op->yf_n1;
+static bool uses_tc(const avx_operator* op, bool base) {
+  return op->kind == 0 && op->dft_mode == AVX_DFT_SPLIT_BF16X3 && op->tc_np > 0 && (base || !op->yf_n1);
 }
 
-static void set_dft(KArgs* k, const avx_operator* op) {
-  k->yf_n1 = op->yf_n1;
+static void set_dft(KArgs* k, const avx_operator* op, bool base = false) {
+  k->yf_n1 = base ? 0 : op->yf_n1;
   k->yf_rows = op->max_rows;
   k->yf_order = op->yf_order.p;
   k->yf_coef = op->yf_coef.p;
-  k->yw_inv = op->yfull ? op->yw_inv.p : nullptr;
+  k->yw_inv = op->yfull && !base ? op->yw_inv.p : nullptr;
   k->yw_phase = op->yw_phase.p;
-  const bool on = uses_tc(op);
+  k->rows_stockham = base;
+  const bool on = uses_tc(op, base);
   k->tc_ytab = on ? op->tc_ytab.p : nullptr;
   k->tc_np = on ? op->tc_np : 0;
   k->tc_ctab = on ? op->tc_ctab.p : nullptr;
   k->tc_kc = on ? op->tc_np : 0;
 }
 
-static KArgs make_kargs(avx_solver* s, const float2* b1, const float2* in, const float2* in2) {
+static KArgs make_kargs(avx_solver* s, const float2* b1, const float2* in, bool base) {
   KArgs k;
   memset(&k, 0, sizeof(k));
   k.g = s->op->geom();
   k.b1 = b1;
   k.in = in;
-  k.in2 = in2;
   k.z = s->z.p;
   k.d = s->d.p;
   k.qp = s->op->d_qp.p;
@@ -982,8 +1057,8 @@ static KArgs make_kargs(avx_solver* s, const float2* b1, const float2* in, const
   k.binary_mask = s->op->binary ? 1 : 0;
   k.st = s->st.p;
   k.partial = s->pk.p;
-  set_dft(&k, s->op);
-  k.b1t = s->b1t.p;
+  set_dft(&k, s->op, base);
+  k.b1t = base ? s->b1t_base.p : s->b1t.p;
   k.rows_kc = s->rows_kc;
   k.rows_rt = s->rows_rt;
   return k;
@@ -991,16 +1066,23 @@ static KArgs make_kargs(avx_solver* s, const float2* b1, const float2* in, const
 
 // the coil maps in the order the operator's y-transforms read them, into buf
 // (left alone when they read the maps as they are)
-static avx_status order_maps(const avx_operator* op, const float2* b1, DevBuf<float2>& buf, cudaStream_t s) {
-  if (op->yf_n1) {
+static avx_status order_maps(const avx_operator* op, const float2* b1, DevBuf<float2>& buf, cudaStream_t s,
+                             bool base = false) {
+  if (op->yf_n1 && !base) {
     AVX_CK(buf.alloc(avx::yfft_maps_count(op->W, op->H, op->C, op->yf_n1)));
     avx::launch_yfft_maps(b1, buf.p, op->W, op->H, op->C, op->yf_n1, s);
-  } else if (uses_tc(op)) {
+  } else if (uses_tc(op, base)) {
     AVX_CK(buf.alloc(avx::b1t_count(op->W, op->H, op->C)));
     avx::launch_b1_tile_transpose(b1, buf.p, op->W, op->H, op->C, s);
   }
   AVX_CK(cudaGetLastError());
   return AVX_OK;
+}
+
+// what the baseline iterations read: the operator's tables, and the coil maps in their order
+static avx_status prepare_baseline(avx_solver* s, const float2* b1) {
+  const avx_status r = ensure_baseline(s->op);
+  return r == AVX_OK ? order_maps(s->op, b1, s->b1t_base, s->stream, true) : r;
 }
 
 static avx::GapConst make_gapconst(avx_solver* s) {
@@ -1029,8 +1111,8 @@ static unsigned shape_launches(int kind, int shape) {
   return 5u + ((shape & 1) ? 5u : 0u) + ((shape & 2) ? 5u : 0u);
 }
 
-static RArgs solver_rargs(avx_solver* s, const float2* b1, const float2* in, const float2* in2) {
-  RArgs r = make_rargs(s->op, b1, in, in2);
+static RArgs solver_rargs(avx_solver* s, const float2* b1, const float2* in, bool base) {
+  RArgs r = make_rargs(s->op, b1, in, nullptr, base);
   r.z = s->z.p;
   r.d = s->d.p;
   r.lam = s->p.lambda;
@@ -1042,9 +1124,9 @@ static RArgs solver_rargs(avx_solver* s, const float2* b1, const float2* in, con
 // radial operator pass: K u (mode 0 z prox, 1 norm, 2 gap sums) and, for modes
 // 0 and 2, K^H z into the operator's K^H z image.  ev (optional) receives
 // events after the forward FFT, the interpolation and the adjoint.
-static void radial_pass(avx_solver* s, int mode, const float2* b1, const float2* in, const float2* in2,
+static void radial_pass(avx_solver* s, int mode, const float2* b1, const float2* in, bool base,
                         cudaEvent_t* ev = nullptr) {
-  RArgs r = solver_rargs(s, b1, in, in2);
+  RArgs r = solver_rargs(s, b1, in, base);
   avx::launch_rad_forward_grid(r, s->stream);
   if (ev) cudaEventRecord(ev[0], s->stream);
   avx::launch_rad_interp(r, mode, s->stream);
@@ -1055,29 +1137,29 @@ static void radial_pass(avx_solver* s, int mode, const float2* b1, const float2*
   if (ev) cudaEventRecord(ev[2], s->stream);
 }
 
-static void enqueue_shape_radial(avx_solver* s, int shape, const float2* b1, const avx::SideStream& side,
+static void enqueue_shape_radial(avx_solver* s, int shape, bool base, const float2* b1, const avx::SideStream& side,
                                  cudaEvent_t* ev) {
   const PDArgs a = make_pdargs(s);
-  const KArgs kdummy = make_kargs(s, b1, s->extc(0), nullptr);
+  const KArgs kdummy = make_kargs(s, b1, s->extc(0), base);
   if (ev) cudaEventRecord(ev[0], s->stream);
   side.fork(s->stream);
   avx::launch_dual(s->method, a, side.side ? side.side : s->stream);
   if (ev) cudaEventRecord(ev[1], s->stream);
-  radial_pass(s, 0, b1, s->extc(0), nullptr, ev ? ev + 2 : nullptr);
+  radial_pass(s, 0, b1, s->extc(0), base, ev ? ev + 2 : nullptr);
   side.join(s->stream);
   avx::launch_primal(s->method, a, s->stream);
   if (ev) cudaEventRecord(ev[5], s->stream);
-  const int nk = avx::radial_interp_blocks(s->op->rg);
+  const int nk = kspace_blocks(s->op, base);
   if (shape & 1) {
     avx::Ptr8 e;
     const int P = method_P(s->method);
     for (int c = 0; c < 8; ++c) e.p[c] = c < P ? s->escrc(c) : nullptr;
     avx::launch_step_img(s->method, a, e, P, s->pimg.p, s->stream);
-    radial_pass(s, 1, b1, s->escrc(0), nullptr);
+    radial_pass(s, 1, b1, s->escrc(0), base);
     avx::launch_step_finalize(a, s->pimg.p, s->pk.p, nk, s->p.sigmaTauRatio, s->stream);
   }
   if (shape & 2) {
-    radial_pass(s, 2, b1, s->primc(0), nullptr);
+    radial_pass(s, 2, b1, s->primc(0), base);
     double* h = s->hist.p;
     const bool ic = method_ic(s->method);
     avx::launch_gap_tail(s->method, a, kdummy, s->pimg.p, s->pk.p, nk, make_gapconst(s), h,
@@ -1085,24 +1167,24 @@ static void enqueue_shape_radial(avx_solver* s, int shape, const float2* b1, con
   }
 }
 
-static void enqueue_shape(avx_solver* s, int shape, const float2* b1, const avx::SideStream& side,
+static void enqueue_shape(avx_solver* s, int shape, bool base, const float2* b1, const avx::SideStream& side,
                           cudaEvent_t* ev = nullptr) {
   if (s->op->kind == 1) {
-    enqueue_shape_radial(s, shape, b1, side, ev);
+    enqueue_shape_radial(s, shape, base, b1, side, ev);
     return;
   }
   const PDArgs a = make_pdargs(s);
-  const KArgs ks = make_kargs(s, b1, s->extc(0), nullptr);
+  const KArgs ks = make_kargs(s, b1, s->extc(0), base);
   avx::launch_iteration(s->method, a, ks, s->op->r_khz.p, s->stream, side, ev);
   if (shape & 1) {
     avx::Ptr8 e;
     const int P = method_P(s->method);
     for (int c = 0; c < 8; ++c) e.p[c] = c < P ? s->escrc(c) : nullptr;
-    const KArgs ke = make_kargs(s, b1, s->escrc(0), nullptr);
+    const KArgs ke = make_kargs(s, b1, s->escrc(0), base);
     avx::launch_step(s->method, a, ke, e, P, s->pimg.p, s->pk.p, s->p.sigmaTauRatio, s->stream);
   }
   if (shape & 2) {
-    const KArgs kx = make_kargs(s, b1, s->primc(0), nullptr);
+    const KArgs kx = make_kargs(s, b1, s->primc(0), base);
     double* h = s->hist.p;
     const bool ic = method_ic(s->method);
     avx::launch_gap(s->method, a, kx, s->op->r_khz.p, s->pimg.p, s->pk.p, make_gapconst(s), h,
@@ -1185,7 +1267,8 @@ static avx_status solver_begin(avx_solver* s, const float2* data, float2* x, con
   }
   r = prepare_run(s, data, x);
   if (r != AVX_OK) return r;
-  r = order_maps(s->op, b1, s->b1t, s->stream);
+  if (baseline_iter(s, 0)) r = prepare_baseline(s, b1);
+  if (r == AVX_OK && !baseline_iter(s, s->p.maxIt)) r = order_maps(s->op, b1, s->b1t, s->stream);
   if (r != AVX_OK) return r;
   if (s->autotune && !s->tuned) {
     r = autotune(s, b1);
@@ -1195,13 +1278,14 @@ static avx_status solver_begin(avx_solver* s, const float2* data, float2* x, con
   }
   if (s->method == AVX_METHOD_ICTGV2 && s->debug) {
     PDArgs a = make_pdargs(s);
-    const KArgs kx = make_kargs(s, b1, s->primc(0), nullptr);
+    const bool base = baseline_iter(s, 0);
+    const KArgs kx = make_kargs(s, b1, s->primc(0), base);
     double* h = s->hist.p;
     if (s->op->kind == 1) {
       a.khz = s->op->r_khz.p;
-      radial_pass(s, 2, b1, s->primc(0), nullptr);
-      avx::launch_gap_tail(s->method, a, kx, s->pimg.p, s->pk.p, avx::radial_interp_blocks(s->op->rg),
-                           make_gapconst(s), h, h + (s->cap + 1), h + 2 * (s->cap + 1), s->cap, 1, s->stream);
+      radial_pass(s, 2, b1, s->primc(0), base);
+      avx::launch_gap_tail(s->method, a, kx, s->pimg.p, s->pk.p, kspace_blocks(s->op, base), make_gapconst(s), h,
+                           h + (s->cap + 1), h + 2 * (s->cap + 1), s->cap, 1, s->stream);
     } else {
       avx::launch_gap(s->method, a, kx, s->op->r_khz.p, s->pimg.p, s->pk.p, make_gapconst(s), h, h + (s->cap + 1),
                       h + 2 * (s->cap + 1), s->cap, 1, s->stream);
@@ -1224,10 +1308,10 @@ static avx_status solver_begin(avx_solver* s, const float2* data, float2* x, con
 }
 
 // The CUDA graph of iteration shape `shape` (bit 0: step rule, bit 1: gap;
-// kChunkShape: kChunk plain iterations), captured at first use on a stream of
-// the solver's own.
-static avx_status solver_graph(avx_solver* s, int shape, const float2* b1) {
-  if (s->gexec[shape]) return AVX_OK;
+// kChunkShape: kChunk plain iterations) with the operator's transforms or the
+// baseline ones, captured at first use on a stream of the solver's own.
+static avx_status solver_graph(avx_solver* s, int shape, bool base, const float2* b1) {
+  if (s->gexec[base][shape]) return AVX_OK;
   if (!s->capture) {
     int least = 0, greatest = 0;
     AVX_CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -1240,12 +1324,12 @@ static avx_status solver_graph(avx_solver* s, int shape, const float2* b1) {
   const cudaStream_t run = s->stream;
   s->stream = s->capture;  // the launches below go to the capture
   if (shape == kChunkShape)
-    for (unsigned i = 0; i < kChunk; ++i) enqueue_shape(s, 0, b1, s->side);
+    for (unsigned i = 0; i < kChunk; ++i) enqueue_shape(s, 0, base, b1, s->side);
   else
-    enqueue_shape(s, shape, b1, s->side);
+    enqueue_shape(s, shape, base, b1, s->side);
   s->stream = run;
   AVX_CK(cudaStreamEndCapture(s->capture, &g));
-  const cudaError_t e = cudaGraphInstantiate(&s->gexec[shape], g, 0);
+  const cudaError_t e = cudaGraphInstantiate(&s->gexec[base][shape], g, 0);
   cudaGraphDestroy(g);
   AVX_CK(e);
   return AVX_OK;
@@ -1258,7 +1342,7 @@ static int next_graph(const avx_solver* s, unsigned k, unsigned k1, unsigned* n)
   *n = 1;
   if (k + kChunk > k1) return iter_shape(s, k);
   for (unsigned i = 0; i < kChunk; ++i)
-    if (iter_shape(s, k + i)) return iter_shape(s, k);
+    if (iter_shape(s, k + i) || baseline_iter(s, k + i) != baseline_iter(s, k)) return iter_shape(s, k);
   *n = kChunk;
   return kChunkShape;
 }
@@ -1268,9 +1352,10 @@ static int next_graph(const avx_solver* s, unsigned k, unsigned k1, unsigned* n)
 static avx_status solver_enqueue(avx_solver* s, const float2* b1, unsigned k0, unsigned k1, unsigned* launches) {
   for (unsigned k = k0, n; k < k1; k += n) {
     const int shape = next_graph(s, k, k1, &n);
-    avx_status r = solver_graph(s, shape, b1);
+    const bool base = baseline_iter(s, k);
+    avx_status r = solver_graph(s, shape, base, b1);
     if (r != AVX_OK) return r;
-    AVX_CK(cudaGraphLaunch(s->gexec[shape], s->stream));
+    AVX_CK(cudaGraphLaunch(s->gexec[base][shape], s->stream));
     if (launches) *launches += n * shape_launches(s->op->kind, shape == kChunkShape ? 0 : shape);
   }
   return AVX_OK;
@@ -1314,7 +1399,7 @@ static avx_status solver_run(avx_solver* s, const float2* data, float2* x, const
     if (s->timing) {
       const int shape = iter_shape(s, k);
       launches += shape_launches(s->op->kind, shape);
-      enqueue_shape(s, shape, b1, avx::SideStream(), &s->events[NEV * k]);
+      enqueue_shape(s, shape, baseline_iter(s, k), b1, avx::SideStream(), &s->events[NEV * k]);
       AVX_CK(cudaGetLastError());
       ++k;
       continue;
@@ -2087,13 +2172,12 @@ avx_status avx_solver_adapt_step_size(avx_solver* s, const avx_cf32* const* d_di
   const float2* b1 = reinterpret_cast<const float2*>(d_b1);
   if (s->op->kind == 1) {
     avx::launch_step_img(s->method, a, e, P, s->pimg.p, s->stream);
-    radial_pass(s, 1, b1, s->escrc(0), nullptr);
-    avx::launch_step_finalize(a, s->pimg.p, s->pk.p, avx::radial_interp_blocks(s->op->rg), s->p.sigmaTauRatio,
-                              s->stream);
+    radial_pass(s, 1, b1, s->escrc(0), false);
+    avx::launch_step_finalize(a, s->pimg.p, s->pk.p, kspace_blocks(s->op, false), s->p.sigmaTauRatio, s->stream);
   } else {
     r = order_maps(s->op, b1, s->b1t, s->stream);
     if (r != AVX_OK) return r;
-    const KArgs ke = make_kargs(s, b1, s->escrc(0), nullptr);
+    const KArgs ke = make_kargs(s, b1, s->escrc(0), false);
     avx::launch_step(s->method, a, ke, e, P, s->pimg.p, s->pk.p, s->p.sigmaTauRatio, s->stream);
   }
   AVX_CK(cudaGetLastError());
@@ -2115,7 +2199,7 @@ avx_status avx_solver_compute_gap(avx_solver* s, const avx_cf32* const* d_x, con
   const size_t N = (size_t)s->N();
   r = prepare_run(s, reinterpret_cast<const float2*>(d_data), nullptr);
   if (r != AVX_OK) return r;
-  r = order_maps(s->op, reinterpret_cast<const float2*>(d_b1), s->b1t, s->stream);
+  r = prepare_baseline(s, reinterpret_cast<const float2*>(d_b1));  // as every reported gap (baseline_iter)
   if (r != AVX_OK) return r;
   for (int c = 0; c < P; ++c)
     AVX_CK(cudaMemcpyAsync(s->primc(c), d_x[c], N * sizeof(float2), cudaMemcpyDeviceToDevice, s->stream));
@@ -2126,16 +2210,15 @@ avx_status avx_solver_compute_gap(avx_solver* s, const avx_cf32* const* d_x, con
   else if (s->op->R)
     avx::launch_gather_rows(s->op->geom(), reinterpret_cast<const float2*>(d_z), s->z.p, 0, s->stream);
   PDArgs a = make_pdargs(s);
-  const KArgs kx = make_kargs(s, reinterpret_cast<const float2*>(d_b1), s->primc(0), nullptr);
+  const KArgs kx = make_kargs(s, reinterpret_cast<const float2*>(d_b1), s->primc(0), true);
   avx::GapConst gc = make_gapconst(s);
   gc.stop_gap = -1.0;
   gc.stop_rel = 0.0;
   double* h = s->hist.p;
-  int nk = s->C * s->T;
+  const int nk = kspace_blocks(s->op, true);
   if (s->op->kind == 1) {
     a.khz = s->op->r_khz.p;
-    nk = avx::radial_interp_blocks(s->op->rg);
-    radial_pass(s, 2, reinterpret_cast<const float2*>(d_b1), s->primc(0), nullptr);
+    radial_pass(s, 2, reinterpret_cast<const float2*>(d_b1), s->primc(0), true);
     avx::launch_gap_tail(s->method, a, kx, s->pimg.p, s->pk.p, nk, gc, h, h + (s->cap + 1), h + 2 * (s->cap + 1),
                          s->cap, 0, s->stream);
   } else {
@@ -2806,6 +2889,8 @@ size_t request_workspace(const avx_request& r, long long R_known, int max_rows_k
     b += T * S * (2 * 4 + 4 + 4) + (W + H) * 4 + sectors * 4 + (Gx + Gy) * c8 + T * C * Gx * Gy * c8 + N * c8;
     b += T * S * (8 + 2 * 8 * 4);  // window starts and Kaiser-Bessel weights
     b += T * S * 4 * 4 + 2 * sectors * 4;  // the spreading's work list, its offsets and order
+    if (r.method == AVX_METHOD_TGV2 || r.method == AVX_METHOD_ICTV)  // the baseline iterations' tables
+      b += T * S * (8 + 2 * 8 * 4 + 4 * 4) + 2 * sectors * 4;
   }
   // solver: primal, extragradient and step scratch (3P), duals (D), z and d, reductions, history
   b += (3 * P + D) * N * c8 + 2 * kspace * c8;
@@ -2865,7 +2950,7 @@ avx_status job_setup(Job* j) {
   // the graphs of every iteration shape the run takes
   for (unsigned k = 0, n; e == AVX_OK && k < j->s->p.maxIt; k += n)
     e = solver_graph(j->s, next_graph(j->s, k, std::min(j->s->p.maxIt, (k / kSlice + 1) * kSlice), &n),
-                     reinterpret_cast<const float2*>(r.d_b1));
+                     baseline_iter(j->s, k), reinterpret_cast<const float2*>(r.d_b1));
   if (e == AVX_OK) {
     const cudaError_t ce = cudaStreamSynchronize(j->stream);
     if (ce != cudaSuccess) e = fail(AVX_E_CUDA, std::string("request set-up: ") + cudaGetErrorString(ce));

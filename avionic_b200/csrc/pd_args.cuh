@@ -76,8 +76,9 @@ struct KArgs {
   // whole two-step y-transforms (null: not used), tables of yfull.cuh
   const int* yw_inv;
   const float2* yw_phase;
-  // row-FFT schedule of the row kernel (chosen by the autotuner): compact rows
-  // per pass (8, 12 or 16; 0 = 16) and the radix plan (0: the compile-time
-  // plan of the length when there is one, 1: the run-time plan)
-  int rows_kc, rows_rt;
+  // schedule of the row kernel: compact rows per pass (8, 12 or 16; 0 = 16) and
+  // its transform.  The two-step split of the length when there is one, unless
+  // rows_stockham asks for Stockham passes (by the compile-time plan of the
+  // length when there is one) or rows_rt for those of the run-time plan
+  int rows_kc, rows_rt, rows_stockham;
 };

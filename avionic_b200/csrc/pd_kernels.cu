@@ -10,6 +10,8 @@
 //   row pass       x-FFT of those rows, z <- prox(z + sigma (K xbar - d)),
 //                  Q' = row-IFFT(mask z): rowfft.cuh, or rows_kernel here for
 //                  widths without a two-step split; one CTA per (coil, frame)
+// (The iterations that baseline_iter of core.cu names run the dense y-transforms
+// of tc_dft.cuh or here and rows_kernel at every size.)
 //   column adjoint K^H z = sum_c conj(b1_c) column-IDFT(Q'_c), by the
 //                  y-transform's form (coladj_kernel here)
 //   primal_kernel  divergence stencils, primal update and extragradient
@@ -619,7 +621,7 @@ __global__ void __launch_bounds__(256, 4) rows_kernel(KArgs a, int mode) {
   constexpr int KCP = AVX_FFT_PITCH(KC);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const CartGeomDev& g = a.g;
-  const int W = g.W, C = g.C;
+  const int W = PLAN > 1 ? PLAN : g.W, C = g.C;  // W compile-time with a fixed plan
   const int c = blockIdx.x % C;
   const int t = blockIdx.x / C;
   const int r0 = g.row_off[t], r1 = g.row_off[t + 1];
@@ -1360,18 +1362,18 @@ void launch_ydft(const KArgs& k, cudaStream_t s) {
 
 template <int KC>
 static void launch_rows_kc(const KArgs& k, int mode, cudaStream_t s) {
-  const int id = fft_plan_id_runtime(k.g.nrad, k.g.rad);
+  // 256 threads, as the compile-time plans assume
+  const int id = k.rows_rt ? fft_plan_id_runtime(k.g.nrad, k.g.rad) : fft_plan_id(k.g.W, k.g.nrad, k.g.rad);
   // launched in plain stream order: as a dependent launch its CTAs, resident early with up to 100 KB of shared
   // memory each, hold up what runs beside them (294 x 24, 4 coils: 50 us an iteration against 31)
 #define CALL_R(ID) rows_kernel<KC, ID><<<k.g.C * k.g.T, 256, rows_smem_bytes(k.g.W, KC), s>>>(k, mode)
-  if (id == 1) CALL_R(1);
-  else CALL_R(0);
+  AVX_FFT_PLAN_DISPATCH(id, CALL_R)
 #undef CALL_R
 }
 
 void launch_rows(const KArgs& k, int mode, cudaStream_t s) {
   int n1, n2;
-  if (!k.rows_rt && rowfft_split(k.g.W, &n1, &n2)) {
+  if (!k.rows_rt && !k.rows_stockham && rowfft_split(k.g.W, &n1, &n2)) {
     launch_rowfft(k, mode, s);
     return;
   }
@@ -1421,8 +1423,8 @@ void launch_iteration(int method, const PDArgs& a, const KArgs& k, float2* khz, 
   // update's stencil little L1) the two only lengthen one another: 84 x 101, 35 frames, 10 coils, 50 rows 308 us
   // an iteration with the dual update beside them, 296 before them; 251 x 174, 46 frames, 4 coils 398 and 327.
   int n1, n2;
-  const SideStream beside =
-      (k.yf_n1 || k.tc_ytab) && !k.rows_rt && rowfft_split(k.g.W, &n1, &n2) ? side : SideStream();
+  const bool rowfft = !k.rows_rt && !k.rows_stockham && rowfft_split(k.g.W, &n1, &n2);
+  const SideStream beside = (k.yf_n1 || k.tc_ytab) && rowfft ? side : SideStream();
   rec(ev, 0, s);
   beside.fork(s);
   launch_dual(method, a, beside.side ? beside.side : s);
@@ -1508,10 +1510,18 @@ cudaError_t configure_kernels() {
   // opt in to the full 227 KB of dynamic shared memory per CTA (sm_100)
   cudaError_t e = cudaFuncSetAttribute(ydft_kernel<KSPACE_KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);
   if (e != cudaSuccess) return e;
-  for (auto f : {rows_kernel<8, 0>, rows_kernel<12, 0>, rows_kernel<KSPACE_KC, 0>, rows_kernel<8, 1>, rows_kernel<12, 1>,
-                 rows_kernel<KSPACE_KC, 1>})
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);
-  return e;
+  for (int id : {96, 128, 160, 192, 256, 320, 1, 0}) {
+#define SET_R(ID)                                                                                                  \
+  e = cudaFuncSetAttribute(rows_kernel<8, ID>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);       \
+  if (e == cudaSuccess)                                                                                            \
+    e = cudaFuncSetAttribute(rows_kernel<12, ID>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);    \
+  if (e == cudaSuccess)                                                                                            \
+    e = cudaFuncSetAttribute(rows_kernel<KSPACE_KC, ID>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX)
+    AVX_FFT_PLAN_DISPATCH(id, SET_R)
+#undef SET_R
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace avx

@@ -173,23 +173,32 @@ __global__ void __launch_bounds__(256) rad_fft_cols_kernel(RArgs a) {
 // index (unwrapped) and weights.  The offsets kappa - g are formed by one
 // fused multiply-add from k: kappa = k G rounded first is off by up to half an
 // ulp of G / 2 (4e-6 grid cells at G = 192), which the window's slope turns
-// into an error of the same order in the weights.
-template <int NW>
+// into an error of the same order in the weights.  ROUNDED: from the rounded
+// kappa all the same, for the baseline iterations (baseline_iter of core.cu).
+template <int NW, bool ROUNDED>
 AVX_D int sample_window(float k, float G, const RadialGeomDev& g, float (&w)[NW]) {
-  const int g0 = (int)floorf(k * G - 0.5f * g.J);
+  if constexpr (ROUNDED) {
+    const float kappa = __fmul_rn(k, G);
+    const int g0 = (int)floorf(kappa - 0.5f * g.J);
 #pragma unroll
-  for (int o = 0; o < NW; ++o) w[o] = kbw(fmaf(k, G, -(float)(g0 + o)), g);
-  return g0;
+    for (int o = 0; o < NW; ++o) w[o] = kbw(kappa - (float)(g0 + o), g);
+    return g0;
+  } else {
+    const int g0 = (int)floorf(k * G - 0.5f * g.J);
+#pragma unroll
+    for (int o = 0; o < NW; ++o) w[o] = kbw(fmaf(k, G, -(float)(g0 + o)), g);
+    return g0;
+  }
 }
 
-template <int NW>
+template <int NW, bool ROUNDED>
 __global__ void rad_window_kernel(RadialGeomDev g, int2* win0, float* winw) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)g.T * g.S;
        i += (long long)gridDim.x * blockDim.x) {
     const int f = (int)(i / g.S), s = (int)(i % g.S);
     float wx[NW], wy[NW];
-    const int g0x = sample_window<NW>(g.traj[((long long)f * 2 + 0) * g.S + s], (float)g.Gx, g, wx);
-    const int g0y = sample_window<NW>(g.traj[((long long)f * 2 + 1) * g.S + s], (float)g.Gy, g, wy);
+    const int g0x = sample_window<NW, ROUNDED>(g.traj[((long long)f * 2 + 0) * g.S + s], (float)g.Gx, g, wx);
+    const int g0y = sample_window<NW, ROUNDED>(g.traj[((long long)f * 2 + 1) * g.S + s], (float)g.Gy, g, wy);
     win0[i] = make_int2(g0x, g0y);
 #pragma unroll
     for (int o = 0; o < NW; ++o) {
@@ -275,7 +284,8 @@ __global__ void __launch_bounds__(256) rad_interp_kernel(RArgs a, int mode) {
   }
 }
 
-// Sectors other than 8 x 8 cells, window widths outside 3 to 5 (else spread.cu):
+// Sectors other than 8 x 8 cells, window widths outside 3 to 5, and the
+// baseline iterations (else spread.cu):
 // one CTA per (sector, frame); thread = grid cell of the sector; CC coils
 // accumulated per pass over the sector's work list: the samples whose window
 // reaches the sector, in the order of the 3x3 neighbouring sectors and of the
@@ -656,9 +666,13 @@ cudaError_t rad_fill_lists(const RadialGeomDev& g, const int* order, const int* 
   return e;
 }
 
-void launch_rad_windows(const RadialGeomDev& g, int2* win0, float* winw, cudaStream_t s) {
+void launch_rad_windows(const RadialGeomDev& g, bool rounded, int2* win0, float* winw, cudaStream_t s) {
   const int nb = (int)std::min<long long>(((long long)g.T * g.S + 255) / 256, 148 * 16);
-#define CALL_W(N) rad_window_kernel<N><<<nb, 256, 0, s>>>(g, win0, winw)
+#define CALL_W(N)                                                     \
+  if (rounded)                                                        \
+    rad_window_kernel<N, true><<<nb, 256, 0, s>>>(g, win0, winw);     \
+  else                                                                \
+    rad_window_kernel<N, false><<<nb, 256, 0, s>>>(g, win0, winw)
   RAD_NW_DISPATCH(g.nw, CALL_W)
 #undef CALL_W
 }

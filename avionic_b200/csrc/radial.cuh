@@ -31,6 +31,7 @@ struct RadialGeomDev {
   int nradx, radx[12];      // FFT plan along x
   int nrady, rady[12];      // FFT plan along y
   int reg_fft;              // the two-step register transforms of radfft.cuh apply
+  int per_sector;           // grid by a block per sector whether or not the half sectors of spread.cuh apply
 };
 
 struct RArgs {
@@ -54,8 +55,9 @@ size_t radial_adj_smem_bytes(int G, int W);
 int radial_interp_blocks(const RadialGeomDev& g);
 cudaError_t configure_radial_kernels();
 
-// per-sample window starts and weights (g.win0, g.winw), once per operator
-void launch_rad_windows(const RadialGeomDev& g, int2* win0, float* winw, cudaStream_t s);
+// per-sample window starts and weights (g.win0, g.winw), once per operator;
+// rounded: from the grid coordinate rounded to fp32 (see sample_window)
+void launch_rad_windows(const RadialGeomDev& g, bool rounded, int2* win0, float* winw, cudaStream_t s);
 // Per-sample tables of an operator, built on the device (stream-ordered, each
 // call returns after its stream work when it reads a result back):
 // flags bit 0: a trajectory value outside [-1/2, 1/2]; bit 1: a negative density

@@ -210,7 +210,7 @@ spread8_kernel(RArgs a, const float2* __restrict__ samples, int items, int heavy
 // Windows of 3 to 5 points are those of kernel widths up to 4; a side of 32 cells keeps a window from reaching a sector
 // from both ends.
 bool spread8_applies(const RadialGeomDev& g) {
-  return g.sw == SW && g.nw >= 3 && g.nw <= 5 && g.Gx >= 32 && g.Gy >= 32;
+  return !g.per_sector && g.sw == SW && g.nw >= 3 && g.nw <= 5 && g.Gx >= 32 && g.Gy >= 32;
 }
 
 template <int NW, int CC>

@@ -5,7 +5,8 @@
 
 namespace avx {
 
-// the grid has sectors of 8 x 8 cells, windows of 3 to 5 points and sides of at least 32 cells
+// the grid has sectors of 8 x 8 cells, windows of 3 to 5 points and sides of at least 32 cells, and g does not ask for
+// a block per sector
 bool spread8_applies(const RadialGeomDev& g);
 // launch_rad_spread of radial.cuh for such a grid
 void launch_spread8(const RArgs& a, const float2* samples, cudaStream_t s);

@@ -1,0 +1,37 @@
+"""Iterations that amplify rounding keep the baseline transforms, bit for bit:
+TGV2 through its step rule at k = 50, ICTV, and runs that report the gap
+history.  Their step sizes are above what the operator's norm allows, so that
+operators which differ by 1e-7 give images 1e-5 to 1e-2 apart, and a gap is a
+difference of sums that agree: the stored values hold one rounding fixed
+(tests/golden/make_baseline_fixtures.py, shapes set, not tuned)."""
+
+import importlib.util
+import os
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+spec = importlib.util.spec_from_file_location("make_baseline_fixtures",
+                                              os.path.join(HERE, "golden", "make_baseline_fixtures.py"))
+fx = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(fx)
+
+
+@pytest.fixture(scope="module")
+def stored():
+    return np.load(os.path.join(HERE, "golden", "baseline", "images.npz"))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", fx.CARTESIAN, ids=fx.name)
+def test_cartesian(stored, case):
+    import avionic_b200 as av
+    assert np.array_equal(fx.cartesian(av, case), stored[fx.name(case)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", fx.RADIAL, ids=fx.name)
+def test_radial(stored, case):
+    import avionic_b200 as av
+    assert np.array_equal(fx.radial(av, case), stored["radial_" + fx.name(case)])
