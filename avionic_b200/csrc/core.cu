@@ -869,15 +869,18 @@ static PDArgs make_pdargs(avx_solver* s) {
 }
 
 // Autotuner of the field-streaming kernels' launch shapes and of the row
-// kernel's FFT schedule.  The first run of a (device, method, W, H, T, C,
-// sampled rows per frame) times every candidate on the solver's own fields
-// (3 warm-up and 5 timed launches each, CUDA events on its stream) and keeps
-// the fastest; later runs and solvers of that shape reuse it.  The trial
-// launches overwrite the fields, so the caller prepares them again.
+// kernel's rows per pass.  The first run of a (device, method, W, H, T, C,
+// sampled rows per frame, transforms) times every candidate on the solver's
+// own fields (launches or operator passes, a few of warm-up and 5 timed, CUDA
+// events on its stream) and keeps the fastest; later runs and solvers of that
+// shape reuse it.  The trial launches overwrite the fields, so the caller
+// prepares them again.
 struct TuneKey {
   int dev, method, W, H, T, C, rows;
+  int transforms;  // the y-transforms in the trial passes
   bool operator<(const TuneKey& o) const {
-    return std::tie(dev, method, W, H, T, C, rows) < std::tie(o.dev, o.method, o.W, o.H, o.T, o.C, o.rows);
+    return std::tie(dev, method, W, H, T, C, rows, transforms) <
+           std::tie(o.dev, o.method, o.W, o.H, o.T, o.C, o.rows, o.transforms);
   }
 };
 // one entry per shape: the map's lock covers lookups only, and each shape's
@@ -887,7 +890,7 @@ struct TuneEntry {
   std::mutex mu;
   bool done = false;
   int primal_tile = 0, dual_block = 0;
-  int rows_kc = KSPACE_KC, rows_rt = 0;
+  int rows_kc = KSPACE_KC;
 };
 static std::mutex g_tune_mu;
 static std::map<TuneKey, std::unique_ptr<TuneEntry>> g_tune;
@@ -911,26 +914,22 @@ static avx_status time_launches(avx_solver* s, void (*launch)(int, const PDArgs&
 
 static KArgs make_kargs(avx_solver* s, const float2* b1, const float2* in, bool base);
 
-// Row-FFT schedules the tuner tries: rows per pass (8, 12, 16) with the
-// compile-time radix plan of the length, and 16 rows per pass with the
-// run-time plan when the length has a compile-time one.  Rows per pass
-// change the schedule only (every sequence goes through the same passes); the
-// two radix plans round differently.
+// Rows per pass that the tuner tries with the row kernel of the run's last
+// iterations: the schedule alone, every sequence goes through the same steps.
+// (The run-time radix plan, which rounds differently, is the caller's to ask
+// for, by avx_solver_set_kspace_schedule: no width has it as the faster one.)
 static avx_status tune_rows(avx_solver* s, const float2* b1) {
   KArgs k = make_kargs(s, b1, s->extc(0), baseline_iter(s, s->p.maxIt));
-  const CartGeomDev& g = k.g;
-  const bool has_fixed = fft_plan_id(g.W, g.nrad, g.rad) != fft_plan_id_runtime(g.nrad, g.rad);
-  const int cand[4][2] = {{KSPACE_KC, 0}, {12, 0}, {8, 0}, {KSPACE_KC, 1}};
-  const int ncand = has_fixed ? 4 : 3;
+  k.rows_rt = 0;
+  s->rows_rt = 0;
   cudaEvent_t e0, e1;
   AVX_CK(cudaEventCreate(&e0));
   AVX_CK(cudaEventCreate(&e1));
   float best = 0.f;
-  for (int i = 0; i < ncand; ++i) {
-    k.rows_kc = cand[i][0];
-    k.rows_rt = cand[i][1];
-    // between its neighbours of an iteration: launches of the row kernel alone overlap one another, which
-    // favours small passes (cine: 8 rows a pass tie with 16 alone, but cost 7 us of an iteration)
+  for (int kc : {KSPACE_KC, 12, 8}) {
+    k.rows_kc = kc;
+    // between its neighbours of an iteration, as dependent launches: alone they overlap one another, which favours
+    // small passes (cine: 8 rows a pass tie with 16 alone, but cost 7 us of an iteration)
     auto chain = [&] {
       avx::launch_ydft(k, s->stream);
       avx::launch_rows(k, 0, s->stream);
@@ -949,10 +948,9 @@ static avx_status tune_rows(avx_solver* s, const float2* b1) {
       cudaEventDestroy(e1);
       return fail(AVX_E_CUDA, std::string("row-schedule tuning: ") + cudaGetErrorString(ce));
     }
-    if (i == 0 || ms < best) {
+    if (kc == KSPACE_KC || ms < best) {
       best = ms;
-      s->rows_kc = cand[i][0];
-      s->rows_rt = cand[i][1];
+      s->rows_kc = kc;
     }
   }
   cudaEventDestroy(e0);
@@ -960,16 +958,11 @@ static avx_status tune_rows(avx_solver* s, const float2* b1) {
   return AVX_OK;
 }
 
-static int max_rows_per_frame(const avx_operator* op) {
-  int m = 0;
-  for (int t = 0; t + 1 < (int)op->row_off.size(); ++t) m = std::max(m, op->row_off[t + 1] - op->row_off[t]);
-  return m;
-}
-
 static avx_status autotune(avx_solver* s, const float2* b1) {
   int dev = 0;
   AVX_CK(cudaGetDevice(&dev));
-  const TuneKey key{dev, s->method, s->W, s->H, s->T, s->C, s->op->kind == 0 ? max_rows_per_frame(s->op) : -1};
+  const TuneKey key{dev,  s->method, s->W, s->H, s->T, s->C, s->op->kind == 0 ? s->op->max_rows : -1,
+                    2 * s->op->dft_mode + (baseline_iter(s, s->p.maxIt) ? 1 : 0)};
   TuneEntry* ent;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -982,31 +975,36 @@ static avx_status autotune(avx_solver* s, const float2* b1) {
     s->primal_tile = ent->primal_tile;
     s->dual_block = ent->dual_block;
     s->rows_kc = ent->rows_kc;
-    s->rows_rt = ent->rows_rt;
+    s->rows_rt = 0;
     s->tuned = true;
     return AVX_OK;
   }
   PDArgs a = make_pdargs(s);
+  a.in_order = 1;
+  // The shapes of one and of two pixels a thread round differently.  Where the iterations amplify that
+  // (baseline_iter: TGV2's images differ by 2.5e-5 after 45), a stopwatch does not choose between them: two pixels
+  // wherever they apply.
+  const bool pairs = avx::dual_pairs(s->method, s->W);
+  const bool only_pairs = pairs && s->method == AVX_METHOD_TGV2;
   float best = 0.f;
-  for (int i = 0; i < AVX_PRIMAL_TILES; ++i) {
-    if (i >= 5 && !avx::dual_pairs(s->method, s->W)) break;
+  const int p0 = only_pairs ? 5 : 0, d0 = only_pairs ? 3 : 0;
+  for (int i = p0; i < (pairs ? AVX_PRIMAL_TILES : 5); ++i) {
     a.primal_tile = i;
     float ms;
     avx_status r = time_launches(s, avx::launch_primal, a, &ms);
     if (r != AVX_OK) return r;
-    if (i == 0 || ms < best) {
+    if (i == p0 || ms < best) {
       best = ms;
       s->primal_tile = i;
     }
   }
   a.primal_tile = s->primal_tile;
-  for (int i = 0; i < AVX_DUAL_BLOCKS; ++i) {
-    if (i >= 3 && !avx::dual_pairs(s->method, s->W)) break;
+  for (int i = d0; i < (pairs ? AVX_DUAL_BLOCKS : 3); ++i) {
     a.dual_block = i;
     float ms;
     avx_status r = time_launches(s, avx::launch_dual, a, &ms);
     if (r != AVX_OK) return r;
-    if (i == 0 || ms < best) {
+    if (i == d0 || ms < best) {
       best = ms;
       s->dual_block = i;
     }
@@ -1019,7 +1017,6 @@ static avx_status autotune(avx_solver* s, const float2* b1) {
   ent->primal_tile = s->primal_tile;
   ent->dual_block = s->dual_block;
   ent->rows_kc = s->rows_kc;
-  ent->rows_rt = s->rows_rt;
   ent->done = true;
   return AVX_OK;
 }

@@ -46,6 +46,7 @@ struct PDArgs {
   const float2* khz;            // K^H z image when the operator supplies it (radial)
   DevState* st;
   int primal_tile, dual_block;  // launch shapes (indices into the tuning tables of pd_kernels.cu)
+  int in_order;                 // dual and primal in plain stream order, not as dependent launches
 };
 
 struct KArgs {

@@ -1273,14 +1273,22 @@ static const int kDualBlocks[AVX_DUAL_BLOCKS] = {256, 128, 512, 256, 128, 512};
 const char* primal_tile_name(int i) { return kPrimalTileNames[(i >= 0 && i < AVX_PRIMAL_TILES) ? i : 0]; }
 int dual_block_threads(int i) { return kDualBlocks[(i >= 0 && i < AVX_DUAL_BLOCKS) ? i : 0]; }
 
+// Trials are launched in order: as dependent launches, runs of one kernel overlap their own copies.
+static void launch_stencil(void (*kernel)(PDArgs), dim3 grid, dim3 block, cudaStream_t s, const PDArgs& a) {
+  if (a.in_order)
+    kernel<<<grid, block, 0, s>>>(a);
+  else
+    launch_dependent(kernel, grid, block, 0, s, a);
+}
+
 template <int NT>
 static void launch_dual_nt(int method, const PDArgs& a, cudaStream_t s) {
   dim3 gd((a.W * a.H + NT - 1) / NT, a.T);
-  if (method == AVX_M_TV) launch_dependent(dual_kernel<AVX_M_TV, NT>, gd, NT, 0, s, a);
-  else if (method == AVX_M_TVTEMP) launch_dependent(dual_kernel<AVX_M_TVTEMP, NT>, gd, NT, 0, s, a);
-  else if (method == AVX_M_TGV2) launch_dependent(dual_kernel<AVX_M_TGV2, NT>, gd, NT, 0, s, a);
-  else if (method == AVX_M_ICTV) launch_dependent(dual_kernel<AVX_M_ICTV, NT>, gd, NT, 0, s, a);
-  else launch_dependent(dual_kernel<AVX_M_ICTGV2, NT>, gd, NT, 0, s, a);
+  if (method == AVX_M_TV) launch_stencil(dual_kernel<AVX_M_TV, NT>, gd, NT, s, a);
+  else if (method == AVX_M_TVTEMP) launch_stencil(dual_kernel<AVX_M_TVTEMP, NT>, gd, NT, s, a);
+  else if (method == AVX_M_TGV2) launch_stencil(dual_kernel<AVX_M_TGV2, NT>, gd, NT, s, a);
+  else if (method == AVX_M_ICTV) launch_stencil(dual_kernel<AVX_M_ICTV, NT>, gd, NT, s, a);
+  else launch_stencil(dual_kernel<AVX_M_ICTGV2, NT>, gd, NT, s, a);
 }
 
 bool dual_pairs(int method, int W) { return (method == AVX_M_TGV2 || method == AVX_M_ICTGV2) && W % 2 == 0; }
@@ -1288,8 +1296,8 @@ bool dual_pairs(int method, int W) { return (method == AVX_M_TGV2 || method == A
 template <int NT>
 static void launch_dual_vec(int method, const PDArgs& a, cudaStream_t s) {
   dim3 gd(((a.W / 2) * a.H + NT - 1) / NT, a.T);
-  if (method == AVX_M_TGV2) launch_dependent(dual_vec_kernel<AVX_M_TGV2, NT>, gd, NT, 0, s, a);
-  else launch_dependent(dual_vec_kernel<AVX_M_ICTGV2, NT>, gd, NT, 0, s, a);
+  if (method == AVX_M_TGV2) launch_stencil(dual_vec_kernel<AVX_M_TGV2, NT>, gd, NT, s, a);
+  else launch_stencil(dual_vec_kernel<AVX_M_ICTGV2, NT>, gd, NT, s, a);
 }
 
 void launch_dual(int method, const PDArgs& a, cudaStream_t s) {
@@ -1312,18 +1320,18 @@ template <int TX, int TY, int YP>
 static void launch_primal_tile(int method, const PDArgs& a, cudaStream_t s) {
   dim3 gp((a.W + TX - 1) / TX, (a.H + TY * YP - 1) / (TY * YP), a.T);
   dim3 bl(TX, TY);
-  if (method == AVX_M_TV) launch_dependent(primal_kernel<AVX_M_TV, TX, TY, YP>, gp, bl, 0, s, a);
-  else if (method == AVX_M_TVTEMP) launch_dependent(primal_kernel<AVX_M_TVTEMP, TX, TY, YP>, gp, bl, 0, s, a);
-  else if (method == AVX_M_TGV2) launch_dependent(primal_kernel<AVX_M_TGV2, TX, TY, YP>, gp, bl, 0, s, a);
-  else if (method == AVX_M_ICTV) launch_dependent(primal_kernel<AVX_M_ICTV, TX, TY, YP>, gp, bl, 0, s, a);
-  else launch_dependent(primal_kernel<AVX_M_ICTGV2, TX, TY, YP>, gp, bl, 0, s, a);
+  if (method == AVX_M_TV) launch_stencil(primal_kernel<AVX_M_TV, TX, TY, YP>, gp, bl, s, a);
+  else if (method == AVX_M_TVTEMP) launch_stencil(primal_kernel<AVX_M_TVTEMP, TX, TY, YP>, gp, bl, s, a);
+  else if (method == AVX_M_TGV2) launch_stencil(primal_kernel<AVX_M_TGV2, TX, TY, YP>, gp, bl, s, a);
+  else if (method == AVX_M_ICTV) launch_stencil(primal_kernel<AVX_M_ICTV, TX, TY, YP>, gp, bl, s, a);
+  else launch_stencil(primal_kernel<AVX_M_ICTGV2, TX, TY, YP>, gp, bl, s, a);
 }
 
 template <int NT>
 static void launch_primal_vec(int method, const PDArgs& a, cudaStream_t s) {
   dim3 gd(((a.W / 2) * a.H + NT - 1) / NT, a.T);
-  if (method == AVX_M_TGV2) launch_dependent(primal_vec_kernel<AVX_M_TGV2, NT>, gd, NT, 0, s, a);
-  else launch_dependent(primal_vec_kernel<AVX_M_ICTGV2, NT>, gd, NT, 0, s, a);
+  if (method == AVX_M_TGV2) launch_stencil(primal_vec_kernel<AVX_M_TGV2, NT>, gd, NT, s, a);
+  else launch_stencil(primal_vec_kernel<AVX_M_ICTGV2, NT>, gd, NT, s, a);
 }
 
 void launch_primal(int method, const PDArgs& a, cudaStream_t s) {
