@@ -836,10 +836,9 @@ void launch_h1_cg(const float2* u, const float2* crec, double mu, int W, int H, 
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (px == 1)
-      cudaLaunchKernelEx(&cfg, h1_cg_resident_kernel<1>, u, crec, mu, W, H, max_it, rel_tol, out, iters, rows);
-    else
-      cudaLaunchKernelEx(&cfg, h1_cg_resident_kernel<2>, u, crec, mu, W, H, max_it, rel_tol, out, iters, rows);
+    auto kernel = px == 1 ? h1_cg_resident_kernel<1> : h1_cg_resident_kernel<2>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaLaunchKernelEx(&cfg, kernel, u, crec, mu, W, H, max_it, rel_tol, out, iters, rows);
     return;
   }
   h1_cg_cluster_kernel<<<C * H1_CLUSTER, 1024, 0, s>>>(u, crec, mu, W, H, max_it, rel_tol, work, muu, out, iters);
@@ -886,13 +885,16 @@ static bool launch_coil_cluster(K (&kernels)[N], const CoilPD& a, int coils, uns
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  const K kernel = kernels[px - 1];
   int fits = 0;
-  if (cudaOccupancyMaxActiveClusters(&fits, kernels[px - 1], &cfg) != cudaSuccess) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&fits, kernel, &cfg) != cudaSuccess) {
     cudaGetLastError();  // a cluster this large cannot be resident on this device
     return false;
   }
   if (fits < 1) return false;
-  if (cudaLaunchKernelEx(&cfg, kernels[px - 1], a, iters, rows) == cudaSuccess) return true;
+  if (cudaLaunchKernelEx(&cfg, kernel, a, iters, rows) == cudaSuccess) return true;
   cudaGetLastError();
   return false;
 }
@@ -913,20 +915,6 @@ bool launch_b1r_cluster(const CoilPD& a, int coils, unsigned iters, cudaStream_t
 bool launch_utgv_cluster(const CoilPD& a, unsigned iters, cudaStream_t s) {
   return launch_coil_cluster(kUtgvCluster, a, 1, iters, 8, 16, s) ||
          launch_coil_cluster(kUtgvCluster, a, 1, iters, 8, 8, s);
-}
-
-cudaError_t configure_coil_kernels() {
-  cudaError_t e = cudaSuccess;
-  auto set = [&](void (*k)(CoilPD, unsigned, int)) {
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  };
-  e = cudaFuncSetAttribute(h1_cg_resident_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(h1_cg_resident_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  for (auto k : kB1Cluster) set(k);
-  for (auto k : kUtgvCluster) set(k);
-  return e;
 }
 
 void launch_b1r_normalize(const float2* x, float2* out, int HW, int coils, cudaStream_t s) {

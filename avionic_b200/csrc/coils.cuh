@@ -64,7 +64,6 @@ void launch_b1r_fused(const CoilPD& a, int coils, const B1Buffers& b, cudaStream
 // in a.x1.
 bool launch_b1r_cluster(const CoilPD& a, int coils, unsigned iters, cudaStream_t s);
 bool launch_utgv_cluster(const CoilPD& a, unsigned iters, cudaStream_t s);
-cudaError_t configure_coil_kernels();
 void launch_b1r_normalize(const float2* x, float2* out, int HW, int coils, cudaStream_t s);
 void launch_phase_apply(const float2* absb1, const float2* x1, float2* out, int HW, cudaStream_t s);
 void launch_weight_update(float2* w, const float2* b, int HW, cudaStream_t s);

@@ -38,6 +38,7 @@
 #include "utils_kernels.cuh"
 #include "radfft.cuh"
 #include "rowfft.cuh"
+#include "spread.cuh"
 #include "yfft.cuh"
 #include "yfull.cuh"
 
@@ -261,7 +262,10 @@ avx_status sum_sq(const float2* v, long long n, cudaStream_t s, double* out) {
   return AVX_OK;
 }
 
-// kernel attributes are per device: one bit per configured device
+// Kernel attributes are per device: one bit per configured device.  The
+// transforms built for many lengths are set where an operator of that length
+// is made: setting loads the kernel, and all of them were 75 ms of every
+// process's first call.
 unsigned long long g_configured = 0;
 
 avx_status configure_once() {
@@ -273,11 +277,6 @@ avx_status configure_once() {
   AVX_CK(avx::configure_radial_kernels());
   AVX_CK(avx::configure_fft2d_kernels());
   AVX_CK(avx::configure_tc_kernels());
-  AVX_CK(avx::configure_yfft_kernels());
-  AVX_CK(avx::configure_yfull_kernels());
-  AVX_CK(avx::configure_rowfft_kernels());
-  AVX_CK(avx::configure_radfft_kernels());
-  AVX_CK(avx::configure_coil_kernels());
   g_configured |= bit;
   return AVX_OK;
 }
@@ -433,6 +432,11 @@ static avx_status build_operator(avx_operator* op, const float* h_mask) {
   op->yf_n1 = max_rows > 0 ? avx::yfull_n1(W, H, T, max_rows) : 0;
   op->yfull = op->yf_n1 != 0;
   if (max_rows > 0 && !op->yfull) op->yf_n1 = avx::yfft_n1(H, max_rows);
+  AVX_CK(avx::configure_rowfft(W));
+  if (op->yfull)
+    AVX_CK(avx::configure_yfull(H));
+  else if (op->yf_n1)
+    AVX_CK(avx::configure_yfft(op->yf_n1));
   if (op->yfull) {
     std::vector<int> inv((size_t)T * H);
     std::vector<float2> phase(H);
@@ -594,6 +598,8 @@ static avx_status build_radial(avx_operator* op, const float* d_traj, const floa
       avx::radial_adj_smem_bytes(g.Gx, W) > AVX_DYN_SMEM_MAX)
     return fail(AVX_E_UNSUPPORTED, "oversampled grid too large for the grid FFT tile");
   g.reg_fft = avx::radfft_applies(g) ? 1 : 0;
+  if (g.reg_fft) AVX_CK(avx::configure_radfft(g));
+  if (avx::spread8_applies(g)) AVX_CK(avx::configure_spread8(g));
   std::vector<float2> twx(g.Gx), twy(g.Gy);
   for (int j = 0; j < g.Gx; ++j) twx[j] = make_float2((float)std::cos(2.0 * M_PI * j / g.Gx), (float)std::sin(2.0 * M_PI * j / g.Gx));
   for (int j = 0; j < g.Gy; ++j) twy[j] = make_float2((float)std::cos(2.0 * M_PI * j / g.Gy), (float)std::sin(2.0 * M_PI * j / g.Gy));

@@ -29,11 +29,11 @@ void launch_radfft_adjoint(const RArgs& a, float2* img, cudaStream_t s) {
   run(a.g.Gy, 3, &a, 0, img, s);
 }
 
-cudaError_t configure_radfft_kernels() {
-  cudaError_t e = radfft_set_a();
-  if (e == cudaSuccess) e = radfft_set_b();
-  if (e == cudaSuccess) e = radfft_set_c();
-  if (e == cudaSuccess) e = radfft_set_d();
+cudaError_t configure_radfft(const RadialGeomDev& g) {
+  cudaError_t e = radfft_set_a(g);
+  if (e == cudaSuccess) e = radfft_set_b(g);
+  if (e == cudaSuccess) e = radfft_set_c(g);
+  if (e == cudaSuccess) e = radfft_set_d(g);
   return e;
 }
 

@@ -432,20 +432,26 @@ void radfft_run(int what, const RArgs& a, int mode, float2* img, cudaStream_t s)
   }
 }
 template <int N1, int N2>
-cudaError_t radfft_set() {
+cudaError_t radfft_set(const RadialGeomDev& g) {
   const cudaFuncAttribute dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t e = cudaFuncSetAttribute(rad_cols_fwd_kernel<N1, N2>, dyn, AVX_DYN_SMEM_MAX);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rad_cols_inv_kernel<N1, N2>, dyn, AVX_DYN_SMEM_MAX);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rad_rows_inv_kernel<N1, N2>, dyn, AVX_DYN_SMEM_MAX);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rad_rows_interp_kernel<N1, N2, 3>, dyn, AVX_DYN_SMEM_MAX);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rad_rows_interp_kernel<N1, N2, 4>, dyn, AVX_DYN_SMEM_MAX);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rad_rows_interp_kernel<N1, N2, 5>, dyn, AVX_DYN_SMEM_MAX);
+  cudaError_t e = cudaSuccess;
+  if (g.Gy == N1 * N2) {
+    e = cudaFuncSetAttribute(rad_cols_fwd_kernel<N1, N2>, dyn, AVX_DYN_SMEM_MAX);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(rad_cols_inv_kernel<N1, N2>, dyn, AVX_DYN_SMEM_MAX);
+  }
+  if (e == cudaSuccess && g.Gx == N1 * N2) {
+    auto interp = g.nw == 4   ? rad_rows_interp_kernel<N1, N2, 4>
+                  : g.nw == 3 ? rad_rows_interp_kernel<N1, N2, 3>
+                              : rad_rows_interp_kernel<N1, N2, 5>;
+    e = cudaFuncSetAttribute(interp, dyn, AVX_DYN_SMEM_MAX);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(rad_rows_inv_kernel<N1, N2>, dyn, AVX_DYN_SMEM_MAX);
+  }
   return e;
 }
 
 #define RADFFT_DECLARE(F)                                                                              \
   bool radfft_run_##F(int G, int what, const RArgs* a, int mode, float2* img, cudaStream_t s);         \
-  cudaError_t radfft_set_##F();                                                                        \
+  cudaError_t radfft_set_##F(const RadialGeomDev& g);                                                  \
   size_t radfft_interp_smem_##F(const RadialGeomDev& g);
 RADFFT_DECLARE(a)
 RADFFT_DECLARE(b)
@@ -458,7 +464,7 @@ RADFFT_DECLARE(d)
 #define RADFFT_SMEM_CASE(N1, N2) \
   case N1 * N2: return rad_interp_smem<N1, N2>(g);
 #define RADFFT_SET_CASE(N1, N2) \
-  if (e == cudaSuccess) e = radfft_set<N1, N2>();
+  if (e == cudaSuccess) e = radfft_set<N1, N2>(g);
 #define RADFFT_DEFINE(F, SPLITS)                                                                       \
   bool radfft_run_##F(int G, int what, const RArgs* a, int mode, float2* img, cudaStream_t s) {        \
     switch (G) { SPLITS(RADFFT_CASE) default: return false; }                                          \
@@ -466,7 +472,7 @@ RADFFT_DECLARE(d)
   size_t radfft_interp_smem_##F(const RadialGeomDev& g) {                                              \
     switch (g.Gx) { SPLITS(RADFFT_SMEM_CASE) default: return 0; }                                      \
   }                                                                                                    \
-  cudaError_t radfft_set_##F() {                                                                       \
+  cudaError_t radfft_set_##F(const RadialGeomDev& g) {                                                 \
     cudaError_t e = cudaSuccess;                                                                       \
     SPLITS(RADFFT_SET_CASE)                                                                            \
     return e;                                                                                          \

@@ -390,8 +390,7 @@ int radial_interp_blocks(const RadialGeomDev& g) {
 }
 
 cudaError_t configure_radial_kernels() {
-  cudaError_t e = configure_spread8_kernels();
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   for (int id : {96, 128, 160, 192, 256, 320, 1, 0}) {
 #define SET_K(ID)                                                                                                   \
   e = cudaFuncSetAttribute(rad_fft_cols_kernel<ID, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX); \

@@ -1,4 +1,4 @@
-// Row transforms of the Cartesian operator with two-step register FFTs (rowfft.cu).
+// Row transforms of the Cartesian operator with two-step register FFTs (rowfft_impl.cuh).
 #pragma once
 
 #include "pd_args.cuh"
@@ -13,6 +13,7 @@ bool rowfft_split(int W, int* n1, int* n2);
 // split; mode 5: Q' = row-IFFT of the sampled rows of the dense k-space in
 // k.dense_in (already masked)
 void launch_rowfft(const KArgs& k, int mode, cudaStream_t s);
-cudaError_t configure_rowfft_kernels();
+// the attributes of length W's kernels (nothing for a length without a split)
+cudaError_t configure_rowfft(int W);
 
 }  // namespace avx

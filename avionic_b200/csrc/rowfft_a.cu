@@ -47,15 +47,26 @@ void launch_rowfft(const KArgs& k, int mode, cudaStream_t s) {
 #undef CALL_W
 }
 
-cudaError_t configure_rowfft_kernels() {
-  cudaError_t (*const all[])() = {rowfft_configure_8,  rowfft_configure_9,  rowfft_configure_10, rowfft_configure_11,
-                                  rowfft_configure_12, rowfft_configure_13, rowfft_configure_14, rowfft_configure_15,
-                                  rowfft_configure_16, rowfft_configure_20, rowfft_configure_short};
-  for (auto f : all) {
-    const cudaError_t e = f();
-    if (e != cudaSuccess) return e;
+cudaError_t configure_rowfft(int W) {
+  int n1 = 0, n2 = 0;
+  if (!rowfft_split(W, &n1, &n2)) return cudaSuccess;
+  if (n2 < 8) return rowfft_configure_short(n1, n2);
+#define CASE_W(N) \
+  case N: return rowfft_configure_##N(n2);
+  switch (n1) {
+    CASE_W(8)
+    CASE_W(9)
+    CASE_W(10)
+    CASE_W(11)
+    CASE_W(12)
+    CASE_W(13)
+    CASE_W(14)
+    CASE_W(15)
+    CASE_W(16)
+    CASE_W(20)
+    default: return cudaSuccess;
   }
-  return cudaSuccess;
+#undef CASE_W
 }
 
 }  // namespace avx

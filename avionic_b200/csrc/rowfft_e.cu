@@ -41,16 +41,15 @@ static void launch_rec(int n1, int n2, const KArgs& k, int mode, cudaStream_t s)
   }
 }
 template <int N1, int N2>
-static cudaError_t configure_rec() {
+static cudaError_t configure_rec(int n1, int n2) {
   if constexpr (N1 <= 16) {
     if constexpr (N2 > 7) {
-      return configure_rec<N1 + 1, 2>();
+      return configure_rec<N1 + 1, 2>(n1, n2);
     } else {
       if constexpr (short_split<N1, N2>()) {
-        const cudaError_t e = rowfft_configure<N1, N2>();
-        if (e != cudaSuccess) return e;
+        if (n1 == N1 && n2 == N2) return rowfft_configure<N1, N2>();
       }
-      return configure_rec<N1, N2 + 1>();
+      return configure_rec<N1, N2 + 1>(n1, n2);
     }
   }
   return cudaSuccess;
@@ -59,6 +58,6 @@ static cudaError_t configure_rec() {
 void rowfft_launch_short(int n1, int n2, const KArgs& k, int mode, cudaStream_t s) {
   launch_rec<5, 2>(n1, n2, k, mode, s);
 }
-cudaError_t rowfft_configure_short() { return configure_rec<5, 2>(); }
+cudaError_t rowfft_configure_short(int n1, int n2) { return configure_rec<5, 2>(n1, n2); }
 
 }  // namespace avx

@@ -235,12 +235,12 @@ cudaError_t rowfft_configure() {
 // lanes idle in one step.
 bool rowfft_short_split(int W, int* n1, int* n2);
 void rowfft_launch_short(int n1, int n2, const KArgs& k, int mode, cudaStream_t s);
-cudaError_t rowfft_configure_short();
+cudaError_t rowfft_configure_short(int n1, int n2);
 
 // one translation unit per first length, so that the instances build in parallel
 #define ROWFFT_DECLARE(N1)                                                       \
   void rowfft_launch_##N1(int n2, const KArgs& k, int mode, cudaStream_t s);     \
-  cudaError_t rowfft_configure_##N1();
+  cudaError_t rowfft_configure_##N1(int n2);
 ROWFFT_DECLARE(8)
 ROWFFT_DECLARE(9)
 ROWFFT_DECLARE(10)
@@ -262,17 +262,14 @@ void rowfft_launch_rec(int n2, const KArgs& k, int mode, cudaStream_t s) {
   }
 }
 template <int N1, int N2>
-cudaError_t rowfft_configure_rec() {
-  if constexpr (N2 >= 8) {
-    const cudaError_t e = rowfft_configure<N1, N2>();
-    return e == cudaSuccess ? rowfft_configure_rec<N1, N2 - 1>() : e;
-  }
+cudaError_t rowfft_configure_rec(int n2) {
+  if constexpr (N2 >= 8) return n2 == N2 ? rowfft_configure<N1, N2>() : rowfft_configure_rec<N1, N2 - 1>(n2);
   return cudaSuccess;
 }
 #define ROWFFT_DEFINE(N1)                                                        \
   void rowfft_launch_##N1(int n2, const KArgs& k, int mode, cudaStream_t s) {    \
     rowfft_launch_rec<N1, (N1 < 16 ? N1 : 16)>(n2, k, mode, s);                  \
   }                                                                              \
-  cudaError_t rowfft_configure_##N1() { return rowfft_configure_rec<N1, (N1 < 16 ? N1 : 16)>(); }
+  cudaError_t rowfft_configure_##N1(int n2) { return rowfft_configure_rec<N1, (N1 < 16 ? N1 : 16)>(n2); }
 
 }  // namespace avx

@@ -255,10 +255,8 @@ static cudaError_t configure() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);
   return e;
 }
-cudaError_t configure_spread8_kernels() {
-  cudaError_t e = configure<3>();
-  if (e == cudaSuccess) e = configure<4>();
-  return e == cudaSuccess ? configure<5>() : e;
+cudaError_t configure_spread8(const RadialGeomDev& g) {
+  return g.nw == 3 ? configure<3>() : g.nw == 4 ? configure<4>() : configure<5>();
 }
 
 }  // namespace avx

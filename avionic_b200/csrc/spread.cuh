@@ -10,6 +10,7 @@ namespace avx {
 bool spread8_applies(const RadialGeomDev& g);
 // launch_rad_spread of radial.cuh for such a grid
 void launch_spread8(const RArgs& a, const float2* samples, cudaStream_t s);
-cudaError_t configure_spread8_kernels();
+// the attributes of the kernels of g's window width
+cudaError_t configure_spread8(const RadialGeomDev& g);
 
 }  // namespace avx

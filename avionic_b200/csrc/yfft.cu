@@ -393,16 +393,14 @@ void launch_yfft_adjoint(const KArgs& k, float2* img, cudaStream_t s) {
 #undef CALL_A
 }
 
-cudaError_t configure_yfft_kernels() {
+cudaError_t configure_yfft(int n1) {
   cudaError_t e = cudaSuccess;
-  for (int n1 = 4; n1 <= 16 && e == cudaSuccess; ++n1) {
 #define SET_Y(N)                                                                                                \
   e = cudaFuncSetAttribute(yfft_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX);       \
   if (e == cudaSuccess)                                                                                          \
     e = cudaFuncSetAttribute(yfft_adj_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, AVX_DYN_SMEM_MAX)
-    YFFT_DISPATCH(n1, SET_Y)
+  YFFT_DISPATCH(n1, SET_Y)
 #undef SET_Y
-  }
   return e;
 }
 

@@ -31,6 +31,7 @@ void launch_yfft_maps(const float2* b1, float2* out, int W, int H, int C, int n1
 // coil combination (launch_ydft / launch_adjoint of pd_kernels.cuh)
 void launch_yfft(const KArgs& k, cudaStream_t s);
 void launch_yfft_adjoint(const KArgs& k, float2* img, cudaStream_t s);
-cudaError_t configure_yfft_kernels();
+// the attributes of n1's kernels
+cudaError_t configure_yfft(int n1);
 
 }  // namespace avx

@@ -16,6 +16,7 @@ void yfull_build(int H, int T, int sy, const int* rows, const int* row_off, int*
 // launch_yfft_maps with n1 = yfull_n1
 void launch_yfull(const KArgs& k, cudaStream_t s);
 void launch_yfull_adjoint(const KArgs& k, float2* img, cudaStream_t s);
-cudaError_t configure_yfull_kernels();
+// the attributes of height H's kernels
+cudaError_t configure_yfull(int H);
 
 }  // namespace avx

@@ -35,9 +35,9 @@ static void run(int what, const KArgs& k, float2* img, cudaStream_t s) {
 void launch_yfull(const KArgs& k, cudaStream_t s) { run(0, k, nullptr, s); }
 void launch_yfull_adjoint(const KArgs& k, float2* img, cudaStream_t s) { run(1, k, img, s); }
 
-cudaError_t configure_yfull_kernels() {
-  const cudaError_t e = yfull_set_a();
-  return e == cudaSuccess ? yfull_set_b() : e;
+cudaError_t configure_yfull(int H) {
+  const cudaError_t e = yfull_set_a(H);
+  return e == cudaSuccess ? yfull_set_b(H) : e;
 }
 
 }  // namespace avx

@@ -205,7 +205,7 @@ cudaError_t yfull_set() {
 #define YFULL_DECLARE(F)                                                                   \
   int yfull_first_##F(int H);                                                              \
   bool yfull_run_##F(int what, const KArgs& k, float2* img, cudaStream_t s);               \
-  cudaError_t yfull_set_##F();
+  cudaError_t yfull_set_##F(int H);
 YFULL_DECLARE(a)
 YFULL_DECLARE(b)
 // heights (and only those whose second step has at most 10 points, see above), in two files
@@ -216,7 +216,7 @@ YFULL_DECLARE(b)
 #define YFULL_CASE(N1, N2) \
   case N1 * N2: yfull_run<N1, N2>(what, k, img, s); return true;
 #define YFULL_SET_CASE(N1, N2) \
-  if (e == cudaSuccess) e = yfull_set<N1, N2>();
+  case N1 * N2: return yfull_set<N1, N2>();
 #define YFULL_DEFINE(F, SPLITS)                                                            \
   int yfull_first_##F(int H) {                                                             \
     switch (H) { SPLITS(YFULL_FIRST_CASE) default: return 0; }                             \
@@ -224,10 +224,8 @@ YFULL_DECLARE(b)
   bool yfull_run_##F(int what, const KArgs& k, float2* img, cudaStream_t s) {              \
     switch (k.g.H) { SPLITS(YFULL_CASE) default: return false; }                           \
   }                                                                                        \
-  cudaError_t yfull_set_##F() {                                                            \
-    cudaError_t e = cudaSuccess;                                                           \
-    SPLITS(YFULL_SET_CASE)                                                                 \
-    return e;                                                                              \
+  cudaError_t yfull_set_##F(int H) {                                                       \
+    switch (H) { SPLITS(YFULL_SET_CASE) default: return cudaSuccess; }                     \
   }
 
 }  // namespace avx
