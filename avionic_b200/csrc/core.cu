@@ -362,9 +362,9 @@ struct avx_operator {
 
 // coefficient tables of the tensor-core transforms (at most 48 rows per frame)
 static avx_status build_tc_tables(avx_operator* op) {
-  const int W = op->W, H = op->H, T = op->T, np = op->tc_np, sx = op->centered ? W / 2 : 0, sy = op->centered ? H / 2 : 0;
+  const int H = op->H, T = op->T, np = op->tc_np, sy = op->centered ? H / 2 : 0;
   std::vector<unsigned short> tab(avx::tc_ytab_bytes(H, T, np) / 2);
-  avx::tc_build_ytab(W, H, T, sx, sy, op->rows.data(), op->row_off.data(), np, tab.data());
+  avx::tc_build_ytab(H, T, sy, op->rows.data(), op->row_off.data(), np, tab.data());
   AVX_CK(op->tc_ytab.alloc(tab.size() * 2 / sizeof(uint4)));
   AVX_CK(cudaMemcpy(op->tc_ytab.p, tab.data(), tab.size() * 2, cudaMemcpyHostToDevice));
   std::vector<unsigned short> ctab(avx::tc_ctab_bytes(H, T, np) / 2);
@@ -1315,12 +1315,12 @@ static avx_status solver_begin(avx_solver* s, const float2* data, float2* x, con
 // baseline ones, captured at first use on a stream of the solver's own.
 static avx_status solver_graph(avx_solver* s, int shape, bool base, const float2* b1) {
   if (s->gexec[base][shape]) return AVX_OK;
-  if (!s->capture) {
-    int least = 0, greatest = 0;
-    AVX_CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    AVX_CK(cudaStreamCreateWithPriority(&s->capture, cudaStreamNonBlocking, greatest));
-    AVX_CK(cudaStreamCreateWithPriority(&s->side.side, cudaStreamNonBlocking, least));
+  int least = 0, greatest = 0;
+  AVX_CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  if (!s->capture) AVX_CK(cudaStreamCreateWithPriority(&s->capture, cudaStreamNonBlocking, greatest));
+  if (!s->side.ev && !(base && s->op->kind == 0)) {  // the Cartesian baseline iterations have no parallel branch
     AVX_CK(cudaEventCreateWithFlags(&s->side.ev, cudaEventDisableTiming));
+    AVX_CK(cudaStreamCreateWithPriority(&s->side.side, cudaStreamNonBlocking, least));
   }
   cudaGraph_t g;
   AVX_CK(cudaStreamBeginCapture(s->capture, cudaStreamCaptureModeThreadLocal));

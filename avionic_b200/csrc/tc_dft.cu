@@ -130,35 +130,55 @@ static double host_bf16_value(unsigned short h) {
   return (double)f;
 }
 
-void tc_build_ytab(int W, int H, int T, int sx, int sy, const int* rows, const int* row_off, int np,
-                   unsigned short* out) {
-  (void)W;
-  (void)sx;
+// The three bf16 pieces of e^{2 pi i j / H} / sqrt(H), j = 0 .. H - 1: the
+// tables' values by their phase (with a sine, a cosine and a split for every
+// entry the two tables of H = 320, 46 frames of 32 rows took 144 ms, 14 here).
+struct SplitRoot {
+  unsigned short re[3], im[3], neg_im[3];
+};
+static std::vector<SplitRoot> split_roots(int H) {
+  auto split = [](double v, unsigned short (&p)[3]) {
+    for (unsigned short& h : p) {
+      h = host_bf16((float)v);
+      v -= host_bf16_value(h);
+    }
+  };
+  const double inv = 1.0 / std::sqrt((double)H);
+  std::vector<SplitRoot> out(H);
+  for (int j = 0; j < H; ++j) {
+    const double ang = 2.0 * M_PI * (double)j / H;
+    split(std::cos(ang) * inv, out[j].re);
+    split(std::sin(ang) * inv, out[j].im);
+    split(-std::sin(ang) * inv, out[j].neg_im);
+  }
+  return out;
+}
+// index of the phase of row ky and image row y
+static int root_index(int ky, int y, int sy, int H) {
+  const long long a1 = ((ky - sy) % H + H) % H, a2 = ((y - sy) % H + H) % H;
+  return (int)((a1 * a2) % H);
+}
+static const SplitRoot kNoRoot = {};  // padding rows
+
+void tc_build_ytab(int H, int T, int sy, const int* rows, const int* row_off, int np, unsigned short* out) {
   const int nst = tc_nstage(H);
   const size_t piece = (size_t)tc_piece_bytes(np) / 2;  // in bf16 elements
-  const double inv = 1.0 / std::sqrt((double)H);
+  const std::vector<SplitRoot> roots = split_roots(H);
   for (int t = 0; t < T; ++t) {
     const int r0 = row_off[t], S = row_off[t + 1] - r0;
     for (int s = 0; s < nst; ++s) {
       unsigned short* base = out + ((size_t)t * nst + s) * 3 * piece;
-      for (int n = 0; n < np; ++n)
-        for (int k = 0; k < TC_KS; ++k) {
-          const int kk = n >> 1, y = (s * TC_KS + k) >> 1;
-          double v = 0.0;
-          if (kk < S && y < H) {
-            const int ky = rows[r0 + kk];
-            const long long a1 = ((ky - sy) % H + H) % H, a2 = ((y - sy) % H + H) % H;
-            const double ang = 2.0 * M_PI * (double)((a1 * a2) % H) / H;
-            const double fr = std::cos(ang) * inv, fi = std::sin(ang) * inv;
-            const bool re_out = (n & 1) == 0, re_in = (k & 1) == 0;
-            v = re_out ? (re_in ? fr : -fi) : (re_in ? fi : fr);
-          }
-          const size_t off = (size_t)(n / 8) * 256 + (k / 8) * 64 + (n % 8) * 8 + (k % 8);  // in elements
-          double r = v;
-          for (int p = 0; p < 3; ++p) {
-            const unsigned short h = host_bf16((float)r);
-            base[p * piece + off] = h;
-            r -= host_bf16_value(h);
+      for (int kk = 0; kk < np / 2; ++kk)
+        for (int k = 0; k < TC_KS; k += 2) {
+          const int n = 2 * kk, y = (s * TC_KS + k) >> 1;
+          const SplitRoot& f = kk < S && y < H ? roots[root_index(rows[r0 + kk], y, sy, H)] : kNoRoot;
+          // elements (n, k), (n, k + 1) and, 8 further on, (n + 1, k), (n + 1, k + 1)
+          unsigned short* o = base + (size_t)(n / 8) * 256 + (k / 8) * 64 + (n % 8) * 8 + (k % 8);
+          for (int p = 0; p < 3; ++p, o += piece) {
+            o[0] = f.re[p];
+            o[1] = f.neg_im[p];
+            o[8] = f.im[p];
+            o[9] = f.re[p];
           }
         }
     }
@@ -401,27 +421,19 @@ void tc_build_ctab(int H, int T, int sy, const int* rows, const int* row_off, in
   const int nty = tc_ytiles(H);
   const size_t piece = (size_t)TC_M * kc;  // elements
   const size_t sbo = (size_t)kc / 8 * 64;  // elements between 8-row groups
-  const double inv = 1.0 / std::sqrt((double)H);
+  const std::vector<SplitRoot> roots = split_roots(H);
   for (int t = 0; t < T; ++t) {
     const int r0 = row_off[t], S = row_off[t + 1] - r0;
     for (int ty = 0; ty < nty; ++ty) {
       unsigned short* base = out + ((size_t)t * nty + ty) * 3 * piece;
       for (int r = 0; r < TC_M; ++r)
-        for (int k = 0; k < kc; ++k) {
+        for (int k = 0; k < kc; k += 2) {
           const int y = ty * TC_M + r, kk = k >> 1;
-          double v = 0.0;
-          if (kk < S && y < H) {
-            const int ky = rows[r0 + kk];
-            const long long a1 = ((ky - sy) % H + H) % H, a2 = ((y - sy) % H + H) % H;
-            const double ang = 2.0 * M_PI * (double)((a1 * a2) % H) / H;
-            v = (k & 1) ? -std::sin(ang) * inv : std::cos(ang) * inv;
-          }
-          const size_t off = (size_t)(r / 8) * sbo + (k / 8) * 64 + (r % 8) * 8 + (k % 8);
-          double rr = v;
-          for (int p = 0; p < 3; ++p) {
-            const unsigned short h = host_bf16((float)rr);
-            base[p * piece + off] = h;
-            rr -= host_bf16_value(h);
+          const SplitRoot& f = kk < S && y < H ? roots[root_index(rows[r0 + kk], y, sy, H)] : kNoRoot;
+          unsigned short* o = base + (size_t)(r / 8) * sbo + (k / 8) * 64 + (r % 8) * 8 + (k % 8);
+          for (int p = 0; p < 3; ++p, o += piece) {
+            o[0] = f.re[p];
+            o[1] = f.neg_im[p];
           }
         }
     }

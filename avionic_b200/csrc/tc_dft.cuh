@@ -31,8 +31,7 @@ AVX_HD int tc_nstage(int H) { return (2 * H + TC_KS - 1) / TC_KS; }  // stages o
 //   B[2kk][2y] = Re F, B[2kk][2y+1] = -Im F, B[2kk+1][2y] = Im F, B[2kk+1][2y+1] = Re F
 // with F[kk][y] = exp(+2 pi i (ky_kk - sy)(y - sy) / H) / sqrt(H).
 size_t tc_ytab_bytes(int H, int T, int np);
-void tc_build_ytab(int W, int H, int T, int sx, int sy, const int* rows, const int* row_off, int np,
-                   unsigned short* out);
+void tc_build_ytab(int H, int T, int sy, const int* rows, const int* row_off, int np, unsigned short* out);
 
 size_t tc_ydft_smem_bytes(int np);
 cudaError_t configure_tc_kernels();
