@@ -250,3 +250,12 @@ def test_row_sums_match_oracle(W, kc):
     assert abs(st.sigma - tr["steps"][-1][0]) < 1e-5 * st.sigma
     assert abs(st.tau - tr["steps"][-1][1]) < 1e-5 * st.tau
     assert abs(st.last_gap - tr["PDGap"][-1]) < 2e-5 * tr["PDGap"][-1]
+
+
+# gridding with several half sectors a warp (9472 sectors and frames or more): the benchmark's 12 coils with the most a
+# warp takes and a last block that is not full, windows of 3 and 5 points
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H,C,T,osf,J", [(66, 64, 12, 251, 1.5, 3.0), (64, 64, 3, 70, 1.5, 2.0),
+                                           (64, 64, 9, 70, 1.5, 4.0)])
+def test_gridding_of_many_sectors_matches_oracle(W, H, C, T, osf, J):
+    test_gridding_matches_oracle(W, H, C, T, 1, osf, J)
