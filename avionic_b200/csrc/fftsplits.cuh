@@ -1,8 +1,9 @@
 // Two-factor splits N1 N2 of the transform lengths the two-step column
 // transforms are built for: those of the oversampled grids of image sizes 64
 // to 160 (the smallest even sizes with factors up to 13 at 1.5 and 2 times),
-// which hold the benchmark's matrix sizes too.  In four lists, one per
-// translation unit.
+// which hold the benchmark's matrix sizes too.  Other grids (above 320: images
+// of more than 160 at 2 times, of more than 213 at 1.5) run the Stockham passes.
+// In four lists, one per translation unit.
 #pragma once
 
 #define FFT_SPLITS_A(X) X(12, 8) X(14, 7) X(10, 10) X(13, 8) X(12, 9) X(11, 10) X(14, 8) X(12, 10) X(14, 9) X(16, 8)

@@ -6,7 +6,8 @@
 namespace avx {
 
 // W = n1 n2 with 8 <= n2 <= n1 <= 16, or n1 = 20, or one of the short splits
-// (rowfft_impl.cuh); false when W has no such split
+// (rowfft_impl.cuh); false when W has no such split (so 216, 234, 252, 270 and
+// 288, which would need n1 = 18, run the Stockham passes)
 bool rowfft_split(int W, int* n1, int* n2);
 
 // the row kernel's work (launch_rows of pd_kernels.cuh) for a length with a

@@ -208,7 +208,8 @@ cudaError_t yfull_set() {
   cudaError_t yfull_set_##F(int H);
 YFULL_DECLARE(a)
 YFULL_DECLARE(b)
-// heights (and only those whose second step has at most 10 points, see above), in two files
+// The heights built, in two files: the splits of fftsplits.cuh whose second step has at most 10 points (see above).
+// Other heights, such as 63, 81 or 135, take the class sums at any number of rows.
 #define YFULL_SPLITS_A(X) X(12, 8) X(14, 7) X(10, 10) X(13, 8) X(12, 9) X(11, 10) X(14, 8) X(12, 10)
 #define YFULL_SPLITS_B(X) X(14, 9) X(16, 8) X(13, 10) X(14, 10) X(15, 10) X(16, 10) X(18, 9) X(20, 10)
 #define YFULL_FIRST_CASE(N1, N2) \
