@@ -742,37 +742,6 @@ def main():
     assert torch.isfinite(torch.view_as_real(x)).all().item()
     err_oracle = vs_oracle("cine_192", x) if instance_seed(rank) == 1 else None
 
-    # the operator's other DFT mode, same problem and schedule (reported beside the headline; at this height both
-    # modes run the fp32 register FFTs, so the images agree)
-    other = None
-    if args.dft == "split" and op.dft_mode == av.DFT_SPLIT_BF16X3:
-        op.dft_mode = av.DFT_FP32
-        for _ in range(2):
-            x.copy_(x0)
-            solver.params = p0
-            solver.run(kd, x, b1)
-        torch.cuda.synchronize()
-        g0, g1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        g0.record()
-        for _ in range(args.steps):
-            x.copy_(x0)
-            solver.params = p0
-            solver.run(kd, x, b1)
-        g1.record()
-        torch.cuda.synchronize()
-        x_fp32 = x.clone()
-        other = {"dft": "fp32", "value": job_rate(world, args.steps, max_over_ranks(dist, g0.elapsed_time(g1), "cuda")),
-                 "unit": UNIT}
-        op.dft_mode = av.DFT_SPLIT_BF16X3
-        x.copy_(x0)
-        solver.params = p0
-        solver.run(kd, x, b1)
-        torch.cuda.synchronize()
-        other["rel_l2_split_vs_fp32"] = float(torch.linalg.vector_norm(x - x_fp32) /
-                                              torch.linalg.vector_norm(x_fp32))
-        if instance_seed(rank) == 1:
-            other["rel_l2_vs_oracle"] = vs_oracle("cine_192", x_fp32)
-
     # per-stage durations: one more reconstruction with CUDA events between the
     # stages of every iteration (kernels launched directly, not from graphs)
     solver.set_timing(True)
@@ -867,7 +836,8 @@ def main():
                                "dual_pixels_per_thread": 2 if tuning[1] >= 3 else 1,
                                "row_fft_rows_per_pass": row_schedule[0],
                                "row_fft_plan": "run-time" if row_schedule[1] else "two-step"},
-                    "dft": args.dft, "other_dft_form": other,
+                    "dft_mode": args.dft,
+                    "y_transform": "fp32 register FFTs (either mode at this height and method)",
                     "recon_latency_ms": {"p50": float(np.percentile(step_ms, 50)),
                                          "p99": float(np.percentile(step_ms, 99))}},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
