@@ -1880,6 +1880,10 @@ avx_status avx_cartesian_operator_create(unsigned width, unsigned height, unsign
   op->W = (int)width; op->H = (int)height; op->C = (int)coils; op->T = (int)frames;
   op->centered = centered ? 1 : 0;
   r = build_operator(op, d_mask ? hm.data() : nullptr);
+  // the applies' copy of the coil maps here, not in their first call (a batch request's operator is not applied)
+  if (r == AVX_OK && op->yf_n1 && !t_pool_stream &&
+      op->b1t.alloc(avx::yfft_maps_count(op->W, op->H, op->C, op->yf_n1)) != cudaSuccess)
+    r = fail(AVX_E_NOMEM, "coil-map buffer of the operator");
   if (r != AVX_OK) {
     delete op;
     return r;
