@@ -208,23 +208,29 @@ avx_status avx_solver_set_stream(avx_solver* s, void* cuda_stream);          /* 
  * the given indices are used.  primal_tile in [0, 7): 32x8x1, 32x4x2, 64x4x1,
  * 32x4x4, 32x16x1 (threads along x, threads along y, pixels per thread along
  * y), then 128 and 256 threads with two pixels per thread and 128-bit
- * accesses (TGV2 and ICTGV2 with an even width; otherwise tile 0); dual_block in [0, 6): 256, 128, 512 threads with one pixel per thread,
+ * accesses (TGV2 and ICTGV2 with an even width; otherwise tile 0);
+ * dual_block in [0, 6): 256, 128, 512 threads with one pixel per thread,
  * then 256, 128, 512 threads with two pixels per thread and 128-bit
  * accesses (TGV2 and ICTGV2 with an even width; otherwise the one-pixel
- * kernel of that block size).  Index 0 is the default shape.  The shapes change the schedule only: every pixel's arithmetic is
- * the same in all of them (results agree to rounding; the compiler may fuse
- * multiply-adds differently in each). */
+ * kernel of that block size).  Index 0 is the default shape.  The shapes
+ * change the schedule only: every pixel's arithmetic is the same in all of
+ * them (results agree to rounding: one and two pixels per thread fuse
+ * multiply-adds differently, which TGV2's first iterations amplify, so its
+ * autotuner takes two pixels wherever they apply). */
 avx_status avx_solver_set_tuning(avx_solver* s, int autotune, int primal_tile, int dual_block);
 /* The shapes in use (chosen by the autotuner after the first run); any output may be NULL. */
 avx_status avx_solver_get_tuning(const avx_solver* s, int* primal_tile, int* dual_block, const char** primal_name,
                                  int* dual_threads);
-/* FFT schedule of the Cartesian operator's row kernel: compact rows per pass
- * (8, 12 or 16; 16 by default) and the radix plan (0: two register steps when
- * the row length has such a split; 1, and other lengths: the run-time plan).  With autotune set (avx_solver_set_tuning) the first run of
- * a (device, method, W, H, T, C, sampled rows per frame) times the candidate
- * schedules on the solver's own fields and keeps the fastest, replacing what
- * is set here.  Rows per pass change the schedule only; the two plans
- * round differently (results agree to fp32 rounding). */
+/* Schedule of the Cartesian operator's row kernel: compact rows per pass (8,
+ * 12 or 16; 16 by default) and the radix plan (0: two register steps when the
+ * row length has such a split; 1, and other lengths: the run-time plan of
+ * Stockham passes).  Iterations that amplify rounding (AVX_DFT_* above) run
+ * Stockham passes with either, with 0 by the compile-time plan of the length
+ * where it has one (96, 128, 160, 192, 256, 320).  With autotune set
+ * (avx_solver_set_tuning) the first run of a shape, sampled rows per frame and
+ * y-transform times the rows per pass on the solver's own fields and keeps the
+ * fastest, with plan 0, replacing what is set here.  Rows per pass change the
+ * schedule only; the plans round differently (results agree to fp32 rounding). */
 avx_status avx_solver_set_kspace_schedule(avx_solver* s, int rows_per_pass, int runtime_plan);
 avx_status avx_solver_get_kspace_schedule(const avx_solver* s, int* rows_per_pass, int* runtime_plan);
 
