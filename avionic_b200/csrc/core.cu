@@ -988,12 +988,14 @@ static avx_status autotune(avx_solver* s, const float2* b1) {
   PDArgs a = make_pdargs(s);
   a.in_order = 1;
   // The shapes of one and of two pixels a thread round differently.  Where the iterations amplify that
-  // (baseline_iter: TGV2's images differ by 2.5e-5 after 45), a stopwatch does not choose between them: two pixels
-  // wherever they apply.
-  const bool pairs = avx::dual_pairs(s->method, s->W);
-  const bool only_pairs = pairs && s->method == AVX_METHOD_TGV2;
+  // (baseline_iter: TGV2's images differ by 2.5e-5 after 45), a stopwatch, which finds them close, does not choose
+  // between them: the primal takes two pixels wherever they apply, the dual from the size on at which its threads
+  // with one pixel each (1280 an SM) are more than one wave (below, four of five processes timed one pixel as the
+  // faster one; at twice that size, none).
+  const bool pairs = avx::dual_pairs(s->method, s->W), fixed = pairs && s->method == AVX_METHOD_TGV2;
+  const bool dual_two = pairs && (!fixed || s->N() > 148 * 1280);
   float best = 0.f;
-  const int p0 = only_pairs ? 5 : 0, d0 = only_pairs ? 3 : 0;
+  const int p0 = fixed ? 5 : 0, d0 = fixed && dual_two ? 3 : 0;
   for (int i = p0; i < (pairs ? AVX_PRIMAL_TILES : 5); ++i) {
     a.primal_tile = i;
     float ms;
@@ -1005,7 +1007,7 @@ static avx_status autotune(avx_solver* s, const float2* b1) {
     }
   }
   a.primal_tile = s->primal_tile;
-  for (int i = d0; i < (pairs ? AVX_DUAL_BLOCKS : 3); ++i) {
+  for (int i = d0; i < (dual_two ? AVX_DUAL_BLOCKS : 3); ++i) {
     a.dual_block = i;
     float ms;
     avx_status r = time_launches(s, avx::launch_dual, a, &ms);

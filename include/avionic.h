@@ -216,7 +216,7 @@ avx_status avx_solver_set_stream(avx_solver* s, void* cuda_stream);          /* 
  * change the schedule only: every pixel's arithmetic is the same in all of
  * them (results agree to rounding: one and two pixels per thread fuse
  * multiply-adds differently, which TGV2's first iterations amplify, so its
- * autotuner takes two pixels wherever they apply). */
+ * autotuner chooses between them by the problem's size alone). */
 avx_status avx_solver_set_tuning(avx_solver* s, int autotune, int primal_tile, int dual_block);
 /* The shapes in use (chosen by the autotuner after the first run); any output may be NULL. */
 avx_status avx_solver_get_tuning(const avx_solver* s, int* primal_tile, int* dual_block, const char** primal_name,
