@@ -319,6 +319,7 @@ struct avx_operator {
   DevBuf<float2> r_twgx, r_twgy, r_grid;
   DevBuf<float2> r_khz;  // K^H z image (T x H x W), both operator kinds
   bool has_mask = false, binary = true;
+  bool weights_above_1 = false;  // some mask value is larger than 1
   std::vector<int> rows, row_off;
   int R = 0;
   double mask_norm2 = 0.0;
@@ -381,6 +382,7 @@ static avx_status build_operator(avx_operator* op, const float* h_mask) {
   op->row_off.assign(T + 1, 0);
   std::vector<float> mrow;
   op->binary = true;
+  op->weights_above_1 = false;
   op->mask_norm2 = 0.0;
   for (int t = 0; t < T; ++t) {
     op->row_off[t] = (int)op->rows.size();
@@ -393,6 +395,7 @@ static avx_status build_operator(avx_operator* op, const float* h_mask) {
           op->mask_norm2 += (double)v * v;
           if (v != 0.f) keep = true;
           if (v != 0.f && v != 1.f) op->binary = false;
+          if (std::fabs(v) > 1.f) op->weights_above_1 = true;
         }
       }
       if (!keep) continue;
@@ -789,14 +792,19 @@ struct avx_solver {
 //    agree again (2e-6 after 500).
 //  - ICTV's step rule leaves out the regulariser (ictv.cpp) and never corrects
 //    them: 1e-4 after 10 iterations, 4e-3 after 200 (160 x 160, 20 frames).
+//  - A mask weight above 1 multiplies the dual variable of its samples once
+//    an iteration (the reference masks its operator's input in place), so
+//    that they grow without bound: 1e-5 after 30 to 100 iterations of any
+//    method (weights of 0.5 to 1.5).
 //  - The reported gap is the difference of sums that come to agree: the split
 //    form's truncation, 2e-6 in a TV image, is 4e-5 in its gap (96 x 96, 450
 //    iterations).
 // A result there is as reproducible as its rounding, so that is not changed
 // for speed.  TV, TVtemp and ICTGV2 (whose rule acts within ten iterations)
-// agree to 1e-5 at most between the two.
+// agree to 5e-6 between the two.
 static bool baseline_iter(const avx_solver* s, unsigned k) {
-  return (s->debug && s->debugstep > 0) || s->method == AVX_METHOD_ICTV || (s->method == AVX_METHOD_TGV2 && k <= 50);
+  return (s->debug && s->debugstep > 0) || s->op->weights_above_1 || s->method == AVX_METHOD_ICTV ||
+         (s->method == AVX_METHOD_TGV2 && k <= 50);
 }
 
 // partial sums of one k-space pass

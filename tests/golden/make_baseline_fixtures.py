@@ -13,9 +13,12 @@ import numpy as np
 
 ROOT = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 
-# method, W, H, iterations, debug step; split (at most 48 sampled rows a frame) and fp32 y-transforms
-CARTESIAN = [("TGV2", 48, 40, 50, 0, "split"), ("TGV2", 40, 36, 45, 0, "fp32"), ("TGV2", 96, 24, 51, 0, "split"),
-             ("ICTV", 40, 36, 30, 0, "split"), ("ICTV", 64, 30, 60, 0, "fp32"), ("TV", 96, 48, 300, 20, "split")]
+# method, W, H, iterations, debug step; split (at most 48 sampled rows a frame) or fp32 y-transforms; mask of 0 and 1 or
+# with weights of 0.5 to 1.5
+CARTESIAN = [("TGV2", 48, 40, 50, 0, "split", "binary"), ("TGV2", 40, 36, 45, 0, "fp32", "binary"),
+             ("TGV2", 96, 24, 51, 0, "split", "binary"), ("ICTV", 40, 36, 30, 0, "split", "binary"),
+             ("ICTV", 64, 30, 60, 0, "fp32", "binary"), ("TV", 96, 48, 300, 20, "split", "binary"),
+             ("TVTEMP", 48, 40, 60, 0, "split", "weighted")]
 RADIAL = [("TGV2", 44, 40, 50), ("ICTV", 48, 44, 20)]
 
 
@@ -26,8 +29,8 @@ def name(case):
 def cartesian(av, case):
     """The image, or the gap history where there is a debug step."""
     from avionic_b200 import synth
-    method, W, H, iters, step, dft = case
-    prob = synth.small(H, H=H, W=W, T=4, C=4)
+    method, W, H, iters, step, dft, weights = case
+    prob = synth.small(H, H=H, W=W, T=4, C=4, binary=weights == "binary")
     op = av.CartesianOperator(W, H, 4, 4, mask=av.to_device(prob["mask"]), centered=False)
     op.dft_mode = av.DFT_SPLIT_BF16X3 if dft == "split" else av.DFT_FP32
     s = av.Solver(method, op)
