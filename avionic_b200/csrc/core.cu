@@ -789,7 +789,10 @@ struct avx_solver {
 //    too small to be seen).  Until then the loop amplifies rounding: two
 //    operators, both within 1e-6 of float64, give images 6e-5 apart after 40
 //    iterations and 2e-4 after 50 (96 x 96, 32 frames, 19 coils), which then
-//    agree again (2e-6 after 500).
+//    agree again: 1.2e-5 after 70 (1e-3 in single pixels), 8e-6 after 100
+//    (1.6e-4), 4e-6 from 130 on, the most of 95 problems.  So the baseline
+//    runs through k = 50 where the run is shorter than 100 iterations or may
+//    be ended by its stop test.
 //  - ICTV's step rule leaves out the regulariser (ictv.cpp) and never corrects
 //    them: 1e-4 after 10 iterations, 4e-3 after 200 (160 x 160, 20 frames).
 //  - A mask weight above 1 multiplies the dual variable of its samples once
@@ -802,9 +805,10 @@ struct avx_solver {
 // A result there is as reproducible as its rounding, so that is not changed
 // for speed.  TV, TVtemp and ICTGV2 (whose rule acts within ten iterations)
 // agree to 5e-6 between the two.
+static bool stop_active(const avx_solver* s) { return s->p.stopPDGap > 0 || s->stop_rel > 0; }
 static bool baseline_iter(const avx_solver* s, unsigned k) {
   return (s->debug && s->debugstep > 0) || s->op->weights_above_1 || s->method == AVX_METHOD_ICTV ||
-         (s->method == AVX_METHOD_TGV2 && k <= 50);
+         (s->method == AVX_METHOD_TGV2 && k <= 50 && (s->p.maxIt < 100 || stop_active(s)));
 }
 
 // partial sums of one k-space pass
@@ -1113,7 +1117,6 @@ static avx::GapConst make_gapconst(avx_solver* s) {
 }
 
 static bool step_due(unsigned k) { return k < 10 || k % 50 == 0; }
-static bool stop_active(const avx_solver* s) { return s->p.stopPDGap > 0 || s->stop_rel > 0; }
 static bool gap_due(const avx_solver* s, unsigned k) {
   return (s->verbose && (k < 10 || k % 50 == 0)) || (s->debug && s->debugstep > 0 && k % (unsigned)s->debugstep == 0) ||
          (stop_active(s) && k % 20 == 0);

@@ -125,8 +125,9 @@ avx_status avx_cartesian_operator_create(unsigned width, unsigned height, unsign
  * whole two-step FFTs, else with the sampled rows' sums over the FFT's
  * classes).  Solver runs whose step sizes amplify rounding keep the dense forms
  * of the mode all the same, so that their images do not move: TGV2 through
- * its first 51 iterations, ICTV, masks with weights above 1, and runs that
- * report the gap (debug export, avx_solver_compute_gap).  The split form needs at
+ * its first 51 iterations in runs of less than 100 or with a stop test, ICTV,
+ * masks with weights above 1, and runs that report the gap (debug export,
+ * avx_solver_compute_gap).  The split form needs at
  * most 48 sampled rows per frame; otherwise AVX_E_UNSUPPORTED is returned and
  * the mode is unchanged.  New operators use the split form when it applies.
  * The radial operator ignores this. */

@@ -1,9 +1,9 @@
 """Iterations that amplify rounding keep the baseline transforms, bit for bit:
-TGV2 through its step rule at k = 50, ICTV, mask weights above 1, and runs that
-report the gap history.  Their step sizes are above what the operator's norm allows, so that
-operators which differ by 1e-7 give images 1e-5 to 1e-2 apart, and a gap is a
-difference of sums that agree: the stored values hold one rounding fixed
-(tests/golden/make_baseline_fixtures.py, shapes set, not tuned)."""
+TGV2 through its step rule at k = 50 in short runs, ICTV, mask weights above 1,
+and runs that report the gap history.  Their step sizes (or weights) are above
+what converges, so that operators which differ by 1e-7 give images 1e-5 to 1e-2
+apart, and a gap is a difference of sums that agree: the stored values hold one
+rounding fixed (tests/golden/make_baseline_fixtures.py, shapes set, not tuned)."""
 
 import importlib.util
 import os
